@@ -12,29 +12,38 @@ template <int PROB, class R, int A>
 size_t inj_smem_t(int threads) {
     return DwStream<R, ProblemOf<PROB, R, A>::type::Mn>::smem_bytes(threads);
 }
+template <int PROB, class R, int A>
+size_t drawn_smem_t(int threads) {
+    return DwStream<R, ProblemOf<PROB, R, A>::type::Mn>::smem_bytes_drawn(threads);
+}
+template <int PROB, class R, int A, int SOLVER, bool INJ>
+constexpr int noise_form() {
+    return INJ ? kCopied : (StepProblem<PROB, R, A, SOLVER>::type::kCarriedChart ? kDrawn : kInline);
+}
 template <int PROB, class R, int A, int SOLVER, bool INJ, int PPT>
 void launch_step_t(const EnsDev* e, const TileDesc* t, int ntiles, int grid, int block, cudaStream_t s) {
-    const size_t dyn = INJ ? inj_smem_t<PROB, R, A>(block / PPT) : 0;
-    step_kernel<PROB, R, A, SOLVER, INJ, PPT><<<grid, block / PPT, dyn, s>>>(e, t, ntiles);
+    constexpr int F = noise_form<PROB, R, A, SOLVER, INJ>();
+    const size_t dyn = F == kCopied ? inj_smem_t<PROB, R, A>(block / PPT) : (F == kDrawn ? drawn_smem_t<PROB, R, A>(block / PPT) : 0);
+    step_kernel<PROB, R, A, SOLVER, F, PPT><<<grid, block / PPT, dyn, s>>>(e, t, ntiles);
 }
 // the injected kernels' staging exceeds the default dynamic shared memory limit: raise it
 // once per device for the largest CTA
-template <int PROB, class R, int A, int SOLVER>
-void prepare_inj_t() {
+template <int PROB, class R, int A, int SOLVER, int F>
+void prepare_ring_t() {
     static std::mutex mu;
     static bool done[64] = {};
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return;
     std::lock_guard<std::mutex> lk(mu);
     if (done[dev]) return;
-    if (cudaFuncSetAttribute(reinterpret_cast<const void*>(&step_kernel<PROB, R, A, SOLVER, true, 1>),
+    if (cudaFuncSetAttribute(reinterpret_cast<const void*>(&step_kernel<PROB, R, A, SOLVER, F, 1>),
                              cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(inj_smem_t<PROB, R, A>(kMaxBlock))) == cudaSuccess)
+                             static_cast<int>(F == kCopied ? inj_smem_t<PROB, R, A>(kMaxBlock) : drawn_smem_t<PROB, R, A>(kMaxBlock))) == cudaSuccess)
         done[dev] = true;
 }
-template <int PROB, class R, int A>
+template <int PROB, class R, int A, int SOLVER>
 void launch_noise_t(const EnsDev* e, int n_ens, int grid, cudaStream_t s) {
-    noise_chunk_kernel<PROB, R, A><<<dim3(static_cast<unsigned>(grid), static_cast<unsigned>(n_ens)), 256, 0, s>>>(e);
+    noise_chunk_kernel<PROB, R, A, sizeof(R) == 8 && (SOLVER == kImplicitMidpoint || SOLVER == kImplicitMidpointExact)><<<dim3(static_cast<unsigned>(grid), static_cast<unsigned>(n_ens)), 256, 0, s>>>(e);
 }
 template <int PROB, class R, int A>
 void launch_init_t(const EnsDev* e, const RawParticles& rp, unsigned long long Np, cudaStream_t s) {
@@ -65,15 +74,18 @@ KernelSet make_set() {
         k.real_bytes = static_cast<int>(sizeof(R));
         k.init = &launch_init_t<PROB, R, A>;
         k.step[0] = &launch_step_t<PROB, R, A, SOLVER, INJ, 1>;
-        k.step_fn[0] = reinterpret_cast<const void*>(&step_kernel<PROB, R, A, SOLVER, INJ, 1>);
+        k.step_fn[0] = reinterpret_cast<const void*>(&step_kernel<PROB, R, A, SOLVER, noise_form<PROB, R, A, SOLVER, INJ>(), 1>);
         if constexpr (sizeof(R) == 4 && !INJ) {  // two particles per thread: FP32, in-kernel noise
             k.step[1] = &launch_step_t<PROB, R, A, SOLVER, INJ, 2>;
-            k.step_fn[1] = reinterpret_cast<const void*>(&step_kernel<PROB, R, A, SOLVER, INJ, 2>);
+            k.step_fn[1] = reinterpret_cast<const void*>(&step_kernel<PROB, R, A, SOLVER, kInline, 2>);
         }
         if constexpr (INJ) {
             k.dyn_smem = &inj_smem_t<PROB, R, A>;
-            k.prepare = &prepare_inj_t<PROB, R, A, SOLVER>;
-            k.noise = &launch_noise_t<PROB, R, A>;
+            k.prepare = &prepare_ring_t<PROB, R, A, SOLVER, kCopied>;
+            if constexpr (sizeof(R) == 8) k.noise = &launch_noise_t<PROB, R, A, SOLVER>;
+        } else if constexpr (noise_form<PROB, R, A, SOLVER, INJ>() == kDrawn) {
+            k.dyn_smem = &drawn_smem_t<PROB, R, A>;
+            k.prepare = &prepare_ring_t<PROB, R, A, SOLVER, kDrawn>;
         }
         k.reduce = &launch_reduce_t<Prob::OUT>;
         k.field = &launch_field_chunk_t<R>;

@@ -8,8 +8,8 @@
 //                   particles per thread: the state lives in registers, each warp
 //                   stages the chunk's B(t) table (computed once per step in FP64 by
 //                   field_chunk_kernel) in shared memory, the Wiener increments come
-//                   from in-kernel Philox (or from HBM in injection mode, staged a few
-//                   steps ahead in shared memory by bulk copies), each step's output sines and
+//                   from in-kernel Philox (inside the step or a few steps ahead in shared
+//                   memory) or from HBM (staged in shared memory by bulk copies), each step's output sines and
 //                   cosines carry to the next step's prepare, and each window's Kahan
 //                   mean is reduced per warp in FP64 and stored in one coalesced store
 //                   (SingleParticleSimulator.h:129-159, MeanSimulationResult.h:87-119)
@@ -19,7 +19,9 @@
 //                   (SingleParticleSimulator.h:236-273)
 #pragma once
 
-#include "sp_physics.cuh"
+#include <type_traits>
+
+#include "sp_physics64.cuh"
 #include "sp_stage.cuh"
 
 namespace sp {
@@ -30,6 +32,12 @@ template <class R, int A> struct ProblemOf<kNeel, R, A> { using type = NeelCart<
 template <class R, int A> struct ProblemOf<kNeelSpherical, R, A> { using type = NeelSph<R, A>; static constexpr int P = param_count_of(kNeelSpherical, A); };
 template <class R, int A> struct ProblemOf<kBrownNeelEuler, R, A> { using type = BrownNeelEuler<R, A>; static constexpr int P = param_count_of(kBrownNeelEuler, A); };
 template <class R, int A> struct ProblemOf<kBrownNeel, R, A> { using type = BrownNeelCart<R, A>; static constexpr int P = param_count_of(kBrownNeel, A); };
+// the form a solver's steps run in: sp_physics64.cuh's for the FP64 explicit steps of the angle problems
+template <int PROB, class R, int A, int SOLVER> struct StepProblem { using type = typename ProblemOf<PROB, R, A>::type; };
+template <int A, int SOLVER> struct StepProblem<kNeelSpherical, double, A, SOLVER> {
+    using type = std::conditional_t<SOLVER == kImplicitMidpoint, NeelSph<double, A>, NeelSphD<A>>;
+};
+template <int A, int SOLVER> struct StepProblem<kBrownNeelEuler, double, A, SOLVER> { using type = BrownNeelEulerD<A>; };
 
 // ------------------------------------------------------------------ FP64 parameter formulas
 constexpr double kBoltzmann = 1.3806485279E-23;  // ParameterCalculatorNeel.h:43
@@ -306,47 +314,63 @@ struct WindowSum<float, OUT> {
 // Resident CTAs of kMaxBlock threads the compiler must allow per SM (0: its own choice,
 // as without the bound; an explicit 1 lets it take up to 255 registers, which made the
 // FP32 kernels 25 % slower at 163-167 registers instead of 128).  The FP64 explicit steps
-// of Brown+Neel Euler/spherical use about 230-255 registers left alone (8 warps per SM, whose FP64
-// dependency chains leave the issue slots idle: the leading stall is `wait`); held to 128
-// registers they spill some state to local memory, which L1 serves, and run 16 warps per
-// SM: 25-31 % more particle-steps/s for an ensemble that fills the GPU (FP64 Millstein,
-// 262144 particles: 9.2e9 against 7.0e9; caps of 96, 112, 144 and 200 registers were
-// slower).  The Brown+Neel Cartesian ones (168-182 registers left alone) gain 12-22 % the
-// same way (Heun, 262144 particles: 2.43e10 against 2.13e10); the Neel kernels need no more
-// than 128 registers anyway.  Of the implicit-midpoint kernels (222-235 registers left
-// alone) the exact-Jacobian one gains 16 % (cubic Neel, 262144 particles: 6.13e9 against
-// 5.27e9) and the reference-matrix one, whose 20 Newton iterations spill more, loses 5 %,
-// so only the former is bound.  Register allocation does not change the arithmetic.
-template <int PROB, class R, int SOLVER, bool INJECT, int PPT>
+// with in-kernel noise are held to 128 registers: left alone they take up to 255, 8 warps per
+// SM, too few to hide the FP64 chains (Brown+Neel Cartesian Heun, 262144 particles: 2.43e10
+// particle-steps/s bound, 2.13e10 not).  Those that read their increments from memory run
+// small ensembles, one or two warps per scheduler, where a spill only lengthens the chain:
+// unbound (Brown+Neel Heun, 1024 particles: 1.70 us per step, 2.79 bound).  Of the
+// implicit-midpoint kernels (222-235 registers left alone) the exact-Jacobian one gains 16 %
+// bound (cubic Neel, 262144 particles: 6.13e9 against 5.27e9) and the reference-matrix one,
+// whose 20 Newton iterations spill more, loses 5 %, so only the former is bound.  Register
+// allocation does not change the arithmetic.
+//
+// Where the increments of a kernel with in-kernel noise are drawn (NOISE): inside the step,
+// where the pairs' chains interleave with the step's own (Cartesian problems, FP32 and the
+// implicit steps), or a stage of steps ahead in a loop of its own (kDrawn, the FP64 angle
+// problems), whose steps fill the registers and the instruction cache by themselves
+// (Neel spherical Euler-Maruyama, 65536 particles: 1.85 us per step staged; Brown+Neel
+// Cartesian Heun, whose step is a third of that: 2.51 inside, 2.85 staged).
+// The angle problems' FP64 steps with the library's sines and pairs called one after another
+// and the chart rotated and turned back on every step: Brown+Neel Millstein, 65536 particles,
+// 9.17 us per step, now 4.10; Heun 12.4, now 5.96.
+template <int PROB, class R, int SOLVER, int NOISE, int PPT>
 constexpr int step_min_blocks() {
-    return (sizeof(R) == 8 && !INJECT && PPT == 1 &&
+    return (sizeof(R) == 8 && NOISE != kCopied &&
             (SOLVER == kEulerMaruyama || SOLVER == kHeun || SOLVER == kMillstein || SOLVER == kEulerMaruyamaNormalized ||
              SOLVER == kImplicitMidpointExact))
                ? 2
                : 0;
 }
-template <int PROB, class R, int A, int SOLVER, bool INJECT, int PPT>
-__global__ void __launch_bounds__(kMaxBlock / PPT, (step_min_blocks<PROB, R, SOLVER, INJECT, PPT>()))
+template <int PROB, class R, int A, int SOLVER, int NOISE, int PPT>
+__global__ void __launch_bounds__(kMaxBlock / PPT, (step_min_blocks<PROB, R, SOLVER, NOISE, PPT>()))
     step_kernel(const EnsDev* __restrict__ ensembles, const TileDesc* __restrict__ tiles, int ntiles) {
-    using Prob = typename ProblemOf<PROB, R, A>::type;
+    using Prob = typename StepProblem<PROB, R, A, SOLVER>::type;
     using St = Stepper<Prob, R, SOLVER>;
     constexpr int D = Prob::D, Mn = Prob::Mn, OUT = Prob::OUT;
     // per-warp copy of the chunk's field table: warps never wait on each other
-    // (a CTA-wide barrier every tile made fast warps wait for slow ones).  Injected kernels
-    // stage 32 steps at a time, leaving shared memory to the increments' ring.
-    constexpr int FT = INJECT ? 32 : kFieldTile;
+    // (a CTA-wide barrier every tile made fast warps wait for slow ones).  Kernels with an
+    // increments' ring stage 32 steps at a time, leaving shared memory to it.
+    constexpr bool kRing = NOISE != kInline;
+    constexpr int FT = kRing ? 32 : kFieldTile;
     __shared__ R sBw[kMaxBlock / 32][FT][3];
     R(*const sB)[3] = sBw[threadIdx.x >> 5];
-    // injection mode: each warp's ring of staged increments (dynamic shared memory)
+    // carried charts: the warp's thresholds (the spherical problem has one chart)
+    __shared__ ChartBounds sCharts[Prob::kCarriedChart ? kMaxBlock / 32 : 1][2];
+    ChartBounds* const charts = sCharts[Prob::kCarriedChart ? threadIdx.x >> 5 : 0];
+    // each warp's ring of increments, copied or drawn (dynamic shared memory)
     using Stream = DwStream<R, Mn>;
-    static_assert(!INJECT || PPT == 1, "injected increments are staged for one particle per thread");
+    constexpr bool kLibraryNoise = SOLVER == kImplicitMidpoint || SOLVER == kImplicitMidpointExact;
+    if constexpr (NOISE != kCopied) load_noise_tables<R>();
+    static_assert(!kRing || PPT == 1, "injected increments are staged for one particle per thread");
     Stream dws;
-    if constexpr (INJECT) {
+    if constexpr (kRing) {
         extern __shared__ __align__(128) unsigned char sp_dyn_smem[];
         __shared__ uint64_t sbar[kMaxBlock / 32][Stream::kStages];
         const int warp = threadIdx.x >> 5;
-        dws.init(reinterpret_cast<R*>(sp_dyn_smem + static_cast<size_t>(warp) * Stream::kStages * Stream::kStageBytes),
-                 sbar[warp]);
+        // the launch sizes the ring: kStages stages per warp (copied increments) or one (drawn)
+        uint32_t dyn;
+        asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn));
+        dws.init(reinterpret_cast<R*>(sp_dyn_smem + static_cast<size_t>(warp) * (dyn / (blockDim.x >> 5))), sbar[warp]);
     }
 
     for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
@@ -379,6 +403,14 @@ __global__ void __launch_bounds__(kMaxBlock / PPT, (step_min_blocks<PROB, R, SOL
         WindowSum<R, OUT> acc[PPT];
         typename Prob::Par q[PPT];
         typename Prob::Trig tr[PPT];  // sincos of y, carried from each step's output to the next prepare
+        if constexpr (Prob::kCarriedChart) {
+            __syncwarp();
+            if ((threadIdx.x & 31) == 0) {
+                charts[0] = chart_bounds(rot.rb, rot.min1, rot.max1);
+                charts[1] = chart_bounds(rot.rn, rot.min2, rot.max2);
+            }
+            __syncwarp();
+        }
 #pragma unroll
         for (int k = 0; k < PPT; ++k) {
             if (active[k]) {
@@ -398,6 +430,10 @@ __global__ void __launch_bounds__(kMaxBlock / PPT, (step_min_blocks<PROB, R, SOL
                 q[k] = Prob::load(static_cast<const R*>(e.params), Np, td.first);  // any valid slot; results are discarded
             }
             Prob::trig(y[k], tr[k]);
+            if constexpr (Prob::kCarriedChart) {
+                Prob::set_chart(active[k] ? e.status[p[k]] : 0, tr[k]);
+                if (s0 == 0) Prob::rechart(charts, y[k], tr[k]);
+            }
             const R* slo = static_cast<const R*>(e.slo);
 #pragma unroll
             for (int i = 0; i < D; ++i) lo[k][i] = (slo && active[k]) ? slo[i * Np + p[k]] : R(0);
@@ -408,10 +444,10 @@ __global__ void __launch_bounds__(kMaxBlock / PPT, (step_min_blocks<PROB, R, SOL
         // live in registers across the step loop.
         unsigned int wpos = static_cast<unsigned int>(s0 % W);
         const unsigned int W32 = static_cast<unsigned int>(W);
-        // injected increments stream from HBM: the warp's rows of the tile's first steps go
+        // copied increments stream from HBM: the warp's rows of the tile's first steps go
         // in flight now (the warp's 32 particles start at the tile's first + 32 warp)
-        if constexpr (INJECT)
-            dws.begin(static_cast<const R*>(e.dw), Np, td.first + (threadIdx.x & ~31u), e.dw_chunk ? 0ull : s0, nsteps);
+        if constexpr (kRing)
+            dws.begin(NOISE == kCopied ? static_cast<const R*>(e.dw) : nullptr, Np, td.first + (threadIdx.x & ~31u), e.dw_chunk ? 0ull : s0, nsteps);
 
         for (unsigned long long t0 = 0; t0 < nsteps; t0 += FT) {
             const int len = static_cast<int>(min(static_cast<unsigned long long>(FT), nsteps - t0));
@@ -427,11 +463,12 @@ __global__ void __launch_bounds__(kMaxBlock / PPT, (step_min_blocks<PROB, R, SOL
                     if (!active[k]) continue;
                     const unsigned long long pid = e.pid_offset + p[k];
                     R w[Mn];
-                    if constexpr (INJECT) {
+                    if constexpr (kRing) {
 #pragma unroll
                         for (int j = 0; j < Mn; ++j) w[j] = winj[k][j];
                     } else {
-                        philox_increments<R, Mn, Prob::kCalledMath>(seed, pid, g, sqdt, m2dt, w);
+                        if constexpr (kLibraryNoise && sizeof(R) == 8) philox_increments_any<Mn>(seed, pid, g, sqdt, w);
+                        else philox_increments<R, Mn>(seed, pid, g, m2dt, w);
                     }
                     if constexpr (SOLVER == kHeunNotConsistent) {
                         R w2[Mn];
@@ -450,6 +487,7 @@ __global__ void __launch_bounds__(kMaxBlock / PPT, (step_min_blocks<PROB, R, SOL
                     }
                     R o[OUT];
                     Prob::out_t(y[k], o, tr[k]);
+                    if constexpr (Prob::kCarriedChart) Prob::rechart(charts, y[k], tr[k]);
                     acc[k].add(o);
                 }
                 if (++wpos == W32) {  // window end: uniform across the CTA
@@ -481,10 +519,23 @@ __global__ void __launch_bounds__(kMaxBlock / PPT, (step_min_blocks<PROB, R, SOL
                     }
                 }
             };
-            if constexpr (INJECT) {
+            if constexpr (kRing) {
+                // in-kernel noise (FP64): a stage of steps is drawn at a time, a small loop of its
+                // own whose independent pairs interleave, instead of inside the step's chain
+                auto draw = [&](R* first, unsigned long long j, int steps) {
+                    if constexpr (NOISE == kDrawn) {
+                        const unsigned long long pid = e.pid_offset + p[0];
+                        for (int st = 0; st < steps; ++st) {
+                            R w[Mn];
+                            philox_increments<R, Mn>(seed, pid, s0 + j + st, m2dt, w);
+#pragma unroll
+                            for (int m = 0; m < Mn; ++m) first[(st * Mn + m) * 32] = w[m];
+                        }
+                    }
+                };
                 for (int i = 0; i < len; ++i) {
                     R cur[PPT][Mn];
-                    if (!dws.next(cur[0])) break;  // a stage timed out (uniform across the warp)
+                    if (!dws.template next<NOISE == kDrawn>(cur[0], draw)) break;  // a stage timed out (uniform across the warp)
                     one_step(i, cur);
                 }
                 if (!dws.ok) break;
@@ -492,7 +543,7 @@ __global__ void __launch_bounds__(kMaxBlock / PPT, (step_min_blocks<PROB, R, SOL
                 for (int i = 0; i < len; ++i) one_step(i, nullptr);
             }
         }
-        if constexpr (INJECT) {
+        if constexpr (kRing) {
             if (!dws.ok) {  // report, wait for the copies still in flight, leave the results unwritten
                 if ((threadIdx.x & 31) == 0) atomicExch(&e.ctl->fault, 1ull);
                 dws.drain();
@@ -518,7 +569,9 @@ __global__ void __launch_bounds__(kMaxBlock / PPT, (step_min_blocks<PROB, R, SOL
                 }
 #pragma unroll
                 for (int c = 0; c < OUT; ++c) { ks[c * Np + p[k]] = acc[k].get_sum(c); kc[c * Np + p[k]] = acc[k].get_comp(c); }
-                if (!finite) e.status[p[k]] = 1;
+                if constexpr (Prob::kCarriedChart)
+                    e.status[p[k]] = static_cast<unsigned char>((e.status[p[k]] & kNonFinite) | (finite ? 0 : kNonFinite) | Prob::chart_bits(tr[k]));
+                else if (!finite) e.status[p[k]] = kNonFinite;
             }
         }
         if constexpr (SOLVER == kImplicitMidpoint || SOLVER == kImplicitMidpointExact) {
@@ -589,10 +642,11 @@ __global__ void field_chunk_kernel(const EnsDev* __restrict__ ensembles, int mid
 // the same Philox counters and the same arithmetic), into dw [chunk][Mn][Np]; the
 // injected step kernel then reads them instead of drawing them on its own step chain.
 // One thread per (step, particle), particles fastest (coalesced stores).
-template <int PROB, class R, int A>
+template <int PROB, class R, int A, bool LIBRARY>
 __global__ void __launch_bounds__(256) noise_chunk_kernel(const EnsDev* __restrict__ ensembles) {
     using Prob = typename ProblemOf<PROB, R, A>::type;
     constexpr int Mn = Prob::Mn;
+    load_noise_tables<R>();
     const EnsDev& e = ensembles[blockIdx.y];
     const unsigned long long s0 = e.ctl->step_done, tgt = e.ctl->step_target;
     const unsigned long long nsteps = tgt > s0 ? min(e.chunk, tgt - s0) : 0ull;
@@ -604,7 +658,8 @@ __global__ void __launch_bounds__(256) noise_chunk_kernel(const EnsDev* __restri
          i += static_cast<unsigned long long>(gridDim.x) * blockDim.x) {
         const unsigned long long j = i / n, p = i - j * n;
         R w[Mn];
-        philox_increments<R, Mn, Prob::kCalledMath>(e.seed, e.pid_offset + p, s0 + j, sqdt, m2dt, w);
+        if constexpr (LIBRARY) philox_increments_any<Mn>(e.seed, e.pid_offset + p, s0 + j, sqdt, w);
+        else philox_increments<R, Mn>(e.seed, e.pid_offset + p, s0 + j, m2dt, w);
 #pragma unroll
         for (int m = 0; m < Mn; ++m) dw[(j * Mn + m) * Np + p] = w[m];
     }
@@ -613,6 +668,7 @@ __global__ void __launch_bounds__(256) noise_chunk_kernel(const EnsDev* __restri
 template <class R, int Mn>
 __global__ void debug_normals_kernel(unsigned long long seed, unsigned long long pid0, unsigned long long n,
                                      unsigned long long step0, unsigned long long nsteps, double* out) {
+    load_noise_tables<R>();
     const unsigned long long idx = static_cast<unsigned long long>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (idx >= n * nsteps) return;
     const unsigned long long s = idx / n, p = idx % n;

@@ -1,6 +1,7 @@
 // sp_math.cuh — precision-generic device math, 3-vectors and the Philox noise source.
 //
-// FP64 instantiations call the IEEE double routines.  FP32 instantiations use
+// FP64 instantiations take their sines, cosines and Box-Muller pairs from sp_fp64.cuh and
+// the rest from the IEEE double routines.  FP32 instantiations use
 // the SFU approximations (__sincosf, __logf) where the stepping tolerates
 // them; the field phase, time and ensemble sums never pass through here in
 // FP32 (they are computed in double by the kernels).
@@ -9,33 +10,18 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "sp_fp64.cuh"
 #include "sp_types.h"
 
 namespace sp {
 
 template <class R> struct M;
 
-// The FP64 step kernels are bound by instruction fetch: every inlined copy of a double
-// transcendental adds a few hundred bytes of code to the step loop.  Their sines and
-// cosines and their Box-Muller pairs are therefore one shared, called routine each
-// (results are those of the same library calls).
-struct SinCosD {
-    double s, c;
-};
-static __device__ __noinline__ SinCosD sincos_d(double x) {
+// the library's sine and cosine, called: every double is an argument
+static __device__ __noinline__ SinCosD sincos_any(double x) {
     SinCosD r;
     ::sincos(x, &r.s, &r.c);
     return r;
-}
-// one Box-Muller pair on the words (a, b): u = (w + 1/2) 2^-32, r = sqrt(-2 ln u_a),
-// (r cos 2 pi u_b, r sin 2 pi u_b)
-static __device__ __noinline__ SinCosD box_muller_pair_d(uint32_t a, uint32_t b) {
-    const double inv = 2.3283064365386963e-10, half = 1.1641532182693481e-10;  // 2^-32, 2^-33
-    const double u0 = fma(static_cast<double>(a), inv, half), u1 = fma(static_cast<double>(b), inv, half);
-    const double r = ::sqrt(-2.0 * ::log(u0));
-    double s, c;
-    ::sincospi(2.0 * u1, &s, &c);
-    return SinCosD{r * s, r * c};
 }
 
 template <> struct M<double> {
@@ -45,7 +31,7 @@ template <> struct M<double> {
     static __device__ __forceinline__ double sin(double x) { return ::sin(x); }
     static __device__ __forceinline__ double cos(double x) { return ::cos(x); }
     static __device__ __forceinline__ void sincos(double x, double* s, double* c) {
-        const SinCosD r = sincos_d(x);
+        const SinCosD r = sincos_any(x);
         *s = r.s;
         *c = r.c;
     }
@@ -153,28 +139,33 @@ __device__ __forceinline__ uint4 philox_block(unsigned long long seed, unsigned 
     return philox4x32_10(c, static_cast<uint32_t>(seed), static_cast<uint32_t>(seed >> 32));
 }
 
-// Box-Muller on u = (w + 1/2) 2^-32.  npairs = 1 or 2 pairs of normals.
-// inlined form, for kernels whose step loop is small enough for the instruction cache
-__device__ __forceinline__ void box_muller_inline(uint4 w, int npairs, double* z) {
-    const double inv = 2.3283064365386963e-10, half = 1.1641532182693481e-10;  // 2^-32, 2^-33
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-        if (k >= npairs) break;
-        const uint32_t a = k ? w.z : w.x, b = k ? w.w : w.y;
-        const double u0 = fma(static_cast<double>(a), inv, half), u1 = fma(static_cast<double>(b), inv, half);
-        const double r = ::sqrt(-2.0 * ::log(u0));
-        double s, c;
-        ::sincospi(2.0 * u1, &s, &c);
-        z[2 * k] = r * c;
-        z[2 * k + 1] = r * s;
+// the logarithm table of the FP64 Box-Muller pairs, in shared memory (128 rows, 3 KB).  Every
+// kernel that draws FP64 normals fills it once, before its first draw, by all threads of the
+// CTA.
+__device__ __forceinline__ LogTab& log_tab() {
+    __shared__ LogTab tab;
+    return tab;
+}
+static __device__ const double kLogTable[kLogRows][3] = {SP_LOG_TABLE};
+template <class R>
+__device__ __forceinline__ void load_noise_tables() {
+    if constexpr (sizeof(R) == 8) {
+        LogTab& t = log_tab();
+        for (int i = threadIdx.x; i < kLogRows; i += blockDim.x) {
+            t.c[i] = kLogTable[i][0];
+            t.l[i][0] = kLogTable[i][1];
+            t.l[i][1] = kLogTable[i][2];
+        }
+        __syncthreads();
     }
 }
+// Box-Muller on u = (w + 1/2) 2^-32.  npairs = 1 or 2 pairs of normals.
 __device__ __forceinline__ void box_muller(uint4 w, int npairs, double* z) {
-    const SinCosD p = box_muller_pair_d(w.x, w.y);
+    const SinCosD p = box_muller_pair(w.x, w.y, -2.0, log_tab());
     z[0] = p.c;
     z[1] = p.s;
     if (npairs > 1) {
-        const SinCosD q = box_muller_pair_d(w.z, w.w);
+        const SinCosD q = box_muller_pair(w.z, w.w, -2.0, log_tab());
         z[2] = q.c;
         z[3] = q.s;
     }
@@ -228,29 +219,51 @@ __device__ __forceinline__ void philox_normals(unsigned long long seed, unsigned
     }
 }
 
-// Wiener increments dW = sqrt(dt) z of one step (m = 3 or 6, calls 0-1).  FP64 scales
-// the unit normals (CALLED: through the shared Box-Muller routine, for kernels whose
-// physics already fills the instruction cache; else inlined, which keeps a small
-// latency-bound step loop free of calls); FP32 folds dt into the Box-Muller radius,
-// sqrt(-2 dt ln u), which saves the m multiplications.
-template <class R, int Mdim, bool CALLED = true>
-__device__ __forceinline__ void philox_increments(unsigned long long seed, unsigned long long pid,
-                                                  unsigned long long step, R sqdt, R m2dt, R* w) {
-    if constexpr (sizeof(R) == 8) {
-        if constexpr (CALLED) {
-            philox_normals<R, Mdim>(seed, pid, step, w);
-        } else {
-            double t[4];
-            box_muller_inline(philox_block(seed, pid, step, 0u), 2, t);
-            w[0] = t[0]; w[1] = t[1]; w[2] = t[2];
-            if (Mdim > 3) {
-                w[3] = t[3];
-                box_muller_inline(philox_block(seed, pid, step, 1u), 1, t);
-                w[4] = t[0]; w[5] = t[1];
-            }
-        }
+// The same increments through the library's logarithm, square root and sine, for the
+// implicit-midpoint steps.  Their Newton iterations (20 with the reference's placeholder
+// Jacobian, which does not converge at the stiff workload's step) amplify an increment's last
+// bit: 65537 cubic particles drift 5e-9 in the mean over 1100 steps when the increments come
+// from box_muller_pair, beyond what an FP64 result may move, and the draw is under 2 % of
+// their step.
+static __device__ __noinline__ SinCosD box_muller_pair_any(uint32_t a, uint32_t b) {
+    const double inv = 2.3283064365386963e-10, half = 1.1641532182693481e-10;  // 2^-32, 2^-33
+    const double u0 = fma(static_cast<double>(a), inv, half), u1 = fma(static_cast<double>(b), inv, half);
+    const double r = ::sqrt(-2.0 * ::log(u0));
+    double s, c;
+    ::sincospi(2.0 * u1, &s, &c);
+    return SinCosD{r * s, r * c};
+}
+template <int Mdim>
+__device__ __forceinline__ void philox_increments_any(unsigned long long seed, unsigned long long pid,
+                                                      unsigned long long step, double sqdt, double* w) {
+    const uint4 a = philox_block(seed, pid, step, 0u);
+    const SinCosD p = box_muller_pair_any(a.x, a.y), q = box_muller_pair_any(a.z, a.w);
+    w[0] = p.c; w[1] = p.s; w[2] = q.c;
+    if (Mdim > 3) {
+        w[3] = q.s;
+        const uint4 b = philox_block(seed, pid, step, 1u);
+        const SinCosD u = box_muller_pair_any(b.x, b.y);
+        w[4] = u.c; w[5] = u.s;
+    }
 #pragma unroll
-        for (int j = 0; j < Mdim; ++j) w[j] = w[j] * sqdt;
+    for (int j = 0; j < Mdim; ++j) w[j] = fp64_mul(w[j], sqdt);
+}
+
+// Wiener increments dW = sqrt(dt) z of one step (m = 3 or 6, calls 0-1).  dt is folded into
+// the Box-Muller radius, sqrt(m2dt ln u) with m2dt = -2 dt, which saves the m multiplications.
+template <class R, int Mdim>
+__device__ __forceinline__ void philox_increments(unsigned long long seed, unsigned long long pid,
+                                                  unsigned long long step, R m2dt, R* w) {
+    if constexpr (sizeof(R) == 8) {
+        const uint4 a = philox_block(seed, pid, step, 0u);
+        const SinCosD p = box_muller_pair(a.x, a.y, m2dt, log_tab()), q = box_muller_pair(a.z, a.w, m2dt, log_tab());
+        w[0] = p.c; w[1] = p.s; w[2] = q.c;
+        if (Mdim > 3) {
+            w[3] = q.s;
+            const uint4 b = philox_block(seed, pid, step, 1u);
+            const SinCosD u = box_muller_pair(b.x, b.y, m2dt, log_tab());
+            w[4] = u.c; w[5] = u.s;
+        }
     } else {
         const float inv = 2.3283064e-10f, half = 1.1641532e-10f;
         const uint4 a = philox_block(seed, pid, step, 0u);

@@ -171,6 +171,7 @@ extern "C" SP_API sp_status sp_simulate_noalloc(const sp_ensemble_desc* desc, co
         rp.K2 = dp.cubic_constant; rp.urot = dp.uniaxial_rotation;
         rp.temperature = desc->temperature;
         rp.simple_model = desc->problem_settings.use_simple_model;
+        if (ks.prepare) ks.prepare();
         ks.init(d_ens, rp, L.Np, s);
         ks.reduce(d_ens, 1, 2, 1, s);
         launches_add(3);  // descriptor and tiles, init, reduce

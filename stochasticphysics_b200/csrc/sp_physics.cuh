@@ -152,7 +152,7 @@ template <class R, int A>
 struct NeelCart {
     static constexpr int D = 3, Mn = 3, OUT = 3;
     static constexpr bool kHasJacobian = true;
-    static constexpr bool kCalledMath = false;  // FP64 Box-Muller through the shared routine
+    static constexpr bool kCarriedChart = false;
     struct Par {
         R NF1, NF2, Dp, pre1, pre2, pF, twoalpha;
         V3<R> z, x, y;
@@ -293,7 +293,7 @@ template <class R, int A>
 struct NeelSph {
     static constexpr int D = 2, Mn = 3, OUT = 3;
     static constexpr bool kHasJacobian = true;
-    static constexpr bool kCalledMath = true;  // FP64 Box-Muller through the shared routine
+    static constexpr bool kCarriedChart = false;
     static constexpr bool kHasExactJacobian = false;
     struct Par {
         R NF1, NF2, Dp, DN, pF, twoalpha;
@@ -524,7 +524,7 @@ template <class R, int A>
 struct BrownNeelEuler {
     static constexpr int D = 5, Mn = 6, OUT = 9;
     static constexpr bool kHasJacobian = false;  // assert(false) in the reference (:605-626)
-    static constexpr bool kCalledMath = true;  // FP64 Box-Muller through the shared routine
+    static constexpr bool kCarriedChart = false;
     static constexpr bool kHasExactJacobian = false;
     struct Par {
         R a, bpd, d, cT, pF, cF, dDN, bpdDN, aDN, adDN2, d2fDN2, cF2h, nd;
@@ -726,30 +726,32 @@ struct BrownNeelEuler {
         const R ctheta = c.C[1], cpsi = c.C[2], spsi = c.S[2];
         const R cos_t = c.C[3], cos_p = c.C[4], sin_t = c.S[3], sin_p = c.S[4];
         const R csc = c.csc;
-        const R cotb = csc * ctheta;
         if (c.br == c.nr) {
-            const R cos_2t = cos_t * cos_t - sin_t * sin_t;
-            const R sin_2t = R(2) * cos_t * sin_t;
-            const R sin_t_2 = sin_t * sin_t;
-            const R cph = cos_p * cpsi + spsi * sin_p;  // cos(phi_N - psi)
-            const R sph = cpsi * sin_p - cos_p * spsi;  // sin(phi_N - psi)
-            // sin and cos of 2 (phi_N - psi) by the double-angle identities
-            const R s2 = R(2) * sph * cph, c2 = cph * cph - sph * sph;
-            r[0] = csc * sin_t * (q.adDN2 * sph - R(2) * q.d2fDN2 * (cos_t * cph + cotb * sin_t * s2));
-            r[1] = q.cF2h * cotb - q.adDN2 * (cph * sin_t) +
-                   q.d2fDN2 * (R(0.5) * (R(3) + cos_2t + R(2) * c2 * sin_t_2) * cotb - sin_2t * sph);
-            r[2] = -(q.adDN2 * (cos_t + sin_t * cotb * sph) -
-                     q.d2fDN2 * sin_t * (R(2) * cos_t * cotb * cph + (R(-1) + R(2) * csc * csc) * sin_t * s2));
+            drift_same(q, csc, ctheta, cpsi, spsi, cos_t, cos_p, sin_t, sin_p, r);
         } else {
-            V3<R> m;
-            if constexpr (M<R>::kColdCalls)
-                m = be_drift_mixed_cold<R>(c.br, q.adDN2, q.d2fDN2, q.cF2h, csc, ctheta, cpsi, spsi, cos_t, cos_p, sin_t, sin_p);
-            else
-                m = be_drift_mixed_impl<R>(c.br, q.adDN2, q.d2fDN2, q.cF2h, csc, ctheta, cpsi, spsi, cos_t, cos_p, sin_t, sin_p);
+            const V3<R> m = be_drift_mixed_impl<R>(c.br, q.adDN2, q.d2fDN2, q.cF2h, csc, ctheta, cpsi, spsi, cos_t, cos_p,
+                                                   sin_t, sin_p);
             r[0] = m.x; r[1] = m.y; r[2] = m.z;
         }
         r[3] = q.nd * c.odst * cos_t;  // :597
         r[4] = R(0);
+    }
+    // the first three components where the charts agree
+    static __device__ __forceinline__ void drift_same(const Par& q, R csc, R ctheta, R cpsi, R spsi, R cos_t, R cos_p,
+                                                      R sin_t, R sin_p, R* r) {
+        const R cotb = csc * ctheta;
+        const R cos_2t = cos_t * cos_t - sin_t * sin_t;
+        const R sin_2t = R(2) * cos_t * sin_t;
+        const R sin_t_2 = sin_t * sin_t;
+        const R cph = cos_p * cpsi + spsi * sin_p;  // cos(phi_N - psi)
+        const R sph = cpsi * sin_p - cos_p * spsi;  // sin(phi_N - psi)
+        // sin and cos of 2 (phi_N - psi) by the double-angle identities
+        const R s2 = R(2) * sph * cph, c2 = cph * cph - sph * sph;
+        r[0] = csc * sin_t * (q.adDN2 * sph - R(2) * q.d2fDN2 * (cos_t * cph + cotb * sin_t * s2));
+        r[1] = q.cF2h * cotb - q.adDN2 * (cph * sin_t) +
+               q.d2fDN2 * (R(0.5) * (R(3) + cos_2t + R(2) * c2 * sin_t_2) * cotb - sin_2t * sph);
+        r[2] = -(q.adDN2 * (cos_t + sin_t * cotb * sph) -
+                 q.d2fDN2 * sin_t * (R(2) * cos_t * cotb * cph + (R(-1) + R(2) * csc * csc) * sin_t * s2));
     }
     // :673-735: x-axis, y-axis, magnetisation
     static __device__ __forceinline__ void out_t(const R* y, R* o, Trig& t) {
@@ -777,7 +779,7 @@ template <class R, int A>
 struct BrownNeelCart {
     static constexpr int D = 6, Mn = 6, OUT = 6;
     static constexpr bool kHasJacobian = true;  // both Jacobians are zero in the reference (.h:119-128)
-    static constexpr bool kCalledMath = false;  // FP64 Box-Muller through the shared routine
+    static constexpr bool kCarriedChart = false;
     static constexpr bool kHasExactJacobian = false;
     struct Par {
         R a, bpd, d, cT, pF, cF, dDN, bpdDN, aDN, cF2, adDN2, hd2DN2, ndrift, cFe;

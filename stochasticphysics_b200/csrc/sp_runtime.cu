@@ -186,13 +186,15 @@ void* Ensemble::dalloc(size_t bytes) {
 }
 
 // Pregenerated noise.  A small ensemble leaves most SMs idle and each step's time is the
-// latency of one thread's step chain, of which the FP64 Philox draw and Box-Muller (double
-// log, sqrt and sincospi) are about half (Neel Heun, 1024 particles: 0.94 us per step with
-// in-kernel noise, 0.43 with the increments read from memory).  With at most two warps per
-// SM scheduler, an FP64 ensemble with in-kernel noise therefore draws each chunk's
+// latency of one thread's step chain, in which the FP64 Philox draw and Box-Muller pairs
+// lengthen the chain (Neel Heun, 1024 particles: 0.67 us per step with in-kernel noise, 0.43
+// with the increments read from memory; Brown+Neel Heun 3.12 and 1.70).  With at most two
+// warps per SM scheduler, an FP64 ensemble with in-kernel noise therefore draws each chunk's
 // increments in a separate, fully parallel kernel (the same Philox counters and
 // arithmetic, so the results are bit-identical) into a chunk-sized buffer that the
-// injected step kernel stages like caller-supplied increments.
+// injected step kernel stages like caller-supplied increments.  At 37888 particles, the
+// limit, Brown+Neel Heun / Millstein take 3.33 / 2.39 us per step against 3.77 / 2.54 drawn
+// in the kernel, Neel Heun 1.03 against 0.83.
 constexpr unsigned long long kPregenWarpsPerSM = 8;  // measured crossover: between 7 and 10
 constexpr unsigned long long kPregenBytes = 256ull << 20;  // cap on the chunk's increments buffer
 
@@ -493,6 +495,32 @@ void reference_times(unsigned long long K, unsigned long long W, double dt, doub
     }
 }
 
+// Angles kept in a rotated chart (status bits, sp_physics64.cuh) to those of the unrotated one
+// (NeelRelaxationSpherical.h:588-602, BrownAndNeelRelaxationEulerSpherical.h:880-899).
+static void unrotate_charts(const sp_ensemble_desc& d, const unsigned char* d_status, size_t n, int D, double* y) {
+    if (d.precision != SP_PRECISION_FP64 ||
+        (d.problem != SP_PROBLEM_NEEL_SPHERICAL && d.problem != SP_PROBLEM_BROWN_AND_NEEL_EULER_SPHERICAL))
+        return;
+    std::vector<unsigned char> bits(n);
+    check_cuda(cudaMemcpy(bits.data(), d_status, n, cudaMemcpyDeviceToHost), "read charts");
+    for (size_t p = 0; p < n; ++p) {
+        double* const a = y + p * D;
+        if (bits[p] & kChartBrown) {
+            const double S0 = std::sin(a[0]), C0 = std::cos(a[0]), S1 = std::sin(a[1]), C1 = std::cos(a[1]),
+                         S2 = std::sin(a[2]), C2 = std::cos(a[2]);
+            a[0] = std::atan2(C0 * C2 - C1 * S0 * S2, -C2 * S0 - C1 * C0 * S2);
+            a[1] = std::acos(S1 * S2);
+            a[2] = std::atan2(-C1, C2 * S1);
+        }
+        if (bits[p] & kChartNeel) {
+            double* const m = a + D - 2;
+            const double st = std::sin(m[0]), ct = std::cos(m[0]), sp = std::sin(m[1]), cp = std::cos(m[1]);
+            m[0] = std::acos(cp * st);
+            m[1] = std::atan2(sp * st, -ct);
+        }
+    }
+}
+
 void Ensemble::read(sp_result* out, sp_stats* st) {
     synchronize();
     EnsCtl ctl;
@@ -537,6 +565,7 @@ void Ensemble::read(sp_result* out, sp_stats* st) {
                     out->final_state[p * L.D + i] =
                         L.real == 8 ? reinterpret_cast<double*>(s.data())[i * L.Np + p]
                                     : static_cast<double>(reinterpret_cast<float*>(s.data())[i * L.Np + p]);
+            unrotate_charts(desc, d_status, L.n, L.D, out->final_state);
         }
     }
     if (st) {
@@ -544,7 +573,7 @@ void Ensemble::read(sp_result* out, sp_stats* st) {
         check_cuda(cudaMemcpy(status.data(), d_status, L.Np, cudaMemcpyDeviceToHost), "read status");
         std::memset(st, 0, sizeof(*st));
         st->particle_steps = particle_steps;
-        for (size_t p = 0; p < L.n; ++p) st->nonfinite_particles += status[p] != 0;
+        for (size_t p = 0; p < L.n; ++p) st->nonfinite_particles += (status[p] & kNonFinite) != 0;
         st->newton_iterations = ctl.newton_iterations;
         st->newton_unconverged = ctl.newton_unconverged;
         st->kernel_launches = launches;

@@ -58,6 +58,9 @@ __device__ __forceinline__ void bulk_copy_g2s(uint32_t dst, const void* src, uin
                  : "memory");
 }
 
+// Kernels that draw their noise a stage at a time use the same buffer, one stage, each lane
+// writing and reading its own column.
+
 // The increments of one warp's 32 particles for the steps of one tile, in order.
 template <class R, int Mn>
 struct DwStream {
@@ -70,6 +73,8 @@ struct DwStream {
 
     // dynamic shared memory of a CTA of `threads` threads
     static constexpr size_t smem_bytes(int threads) { return static_cast<size_t>(threads / 32) * kStages * kStageBytes; }
+    // drawn in the kernel: one stage per warp
+    static constexpr size_t smem_bytes_drawn(int threads) { return static_cast<size_t>(threads / 32) * kStageBytes; }
 
     R* buf;               // this warp's ring: [kStages][kStep][Mn][32]
     uint32_t bar0;        // its first barrier (8 bytes apart)
@@ -118,7 +123,8 @@ struct DwStream {
         Np = np;
         nsteps = n;
         pos = 0;
-        src = dw + s0 * Mn * np + first;
+        src = dw ? dw + s0 * Mn * np + first : nullptr;
+        if (!dw) return;  // drawn, not copied
         const unsigned long long stages = (n + kStep - 1) / kStep;
         for (unsigned long long k = 0; k < stages && k < kStages; ++k) issue(k);
     }
@@ -134,8 +140,19 @@ struct DwStream {
 
     // the increments of the next step for this lane's particle; false once a stage has
     // timed out (uniform across the warp)
-    __device__ __forceinline__ bool next(R* w) {
+    // draw(first, j, steps): writes the increments of steps j .. j + steps - 1 of the tile to
+    // first[(s Mn + m) 32]
+    template <bool DRAWN, class Draw>
+    __device__ __forceinline__ bool next(R* w, Draw draw) {
         const int within = static_cast<int>(pos % kStep);
+        if constexpr (DRAWN) {  // this lane's own draws, the whole stage at once
+            if (within == 0) draw(buf + (threadIdx.x & 31), pos, static_cast<int>(min(static_cast<unsigned long long>(kStep), nsteps - pos)));
+            const R* own = buf + within * Mn * 32 + (threadIdx.x & 31);
+#pragma unroll
+            for (int m = 0; m < Mn; ++m) w[m] = own[m * 32];
+            ++pos;
+            return true;
+        }
         const int slot = static_cast<int>(q_done % kStages);
         if (within == 0) {
             const bool mine = mbar_wait_bounded(bar0 + 8 * slot, (q_done / kStages) & 1u);

@@ -52,6 +52,14 @@ __host__ __device__ constexpr int param_count_of(int problem, int aniso) {
                                         : kParamsBrownNeel;
 }
 
+// bits of a particle's status byte: non-finite state; the FP64 explicit steps of the angle
+// problems also keep which charts the stored angles are those of (sp_physics64.cuh)
+constexpr unsigned char kNonFinite = 1, kChartBrown = 2, kChartNeel = 4;
+
+// where a step kernel's Wiener increments come from: drawn inside the step; copied from the
+// ensemble's dw into a shared-memory ring; drawn into that ring a few steps at a time
+enum NoiseForm : int { kInline = 0, kCopied = 1, kDrawn = 2 };
+
 struct FieldParams {
     int type;  // sp_field_type
     int pad;
@@ -99,7 +107,7 @@ struct EnsDev {
     void* slo;      // FP32 form: [D][Np] carried rounding errors of the state (nullptr in FP64)
     const void* params;
     const double* moment;
-    void* dw;       // Wiener increments [rows][Mn][Np]: injected (every step) or pregenerated
+    void* dw;       // (nullptr: drawn in the step kernel) Wiener increments [rows][Mn][Np]: injected (every step) or pregenerated
     int dw_chunk;   // 1: dw holds only the current chunk's increments (row 0 = its first step)
     double* partial;
     double* msum;   // [K][OUT] weighted ensemble sums
