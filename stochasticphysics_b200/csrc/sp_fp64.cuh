@@ -307,15 +307,27 @@ SP_HD double sqrt_normal(double x) {
     return fma(fma(-g, g, x), h, g);
 }
 
-// 1/x of the sine of an angle, 0 for x = 0 (and for a subnormal x, whose reciprocal only
-// overflows what it multiplies): a third-order step from the hardware's approximation and a
-// residual correction, without the division's branch for special operands
-SP_HD double rcp_or_zero(double x) {
+// 1/x of a normal x: a third-order step from the hardware's approximation and a residual
+// correction, without the division's branch for special operands
+SP_HD double rcp_normal(double x) {
     double y = fp64_rcp_seed(x);
     double e = fma(-x, y, 1.0);
     y = fma(y, fma(e, e, e), y);
     e = fma(-x, y, 1.0);
-    y = fma(y, e, y);
+    return fma(y, e, y);
+}
+
+// a / b from b's reciprocal: quotient and residual correction (P. Markstein, IBM J. Res. Dev.
+// 34, 1990).  The correctly rounded quotient where nothing over- or underflows.
+SP_HD double quotient(double a, double b, double reciprocal) {
+    const double q = fp64_mul(a, reciprocal);
+    return fma(fma(-b, q, a), reciprocal, q);
+}
+
+// 1/x of the sine of an angle, 0 for x = 0 (and for a subnormal x, whose reciprocal only
+// overflows what it multiplies)
+SP_HD double rcp_or_zero(double x) {
+    const double y = rcp_normal(x);
     return (fp64_hi(x) & 0x7ff00000) == 0 ? 0.0 : y;
 }
 

@@ -318,11 +318,10 @@ struct WindowSum<float, OUT> {
 // SM, too few to hide the FP64 chains (Brown+Neel Cartesian Heun, 262144 particles: 2.43e10
 // particle-steps/s bound, 2.13e10 not).  Those that read their increments from memory run
 // small ensembles, one or two warps per scheduler, where a spill only lengthens the chain:
-// unbound (Brown+Neel Heun, 1024 particles: 1.70 us per step, 2.79 bound).  Of the
-// implicit-midpoint kernels (222-235 registers left alone) the exact-Jacobian one gains 16 %
-// bound (cubic Neel, 262144 particles: 6.13e9 against 5.27e9) and the reference-matrix one,
-// whose 20 Newton iterations spill more, loses 5 %, so only the former is bound.  Register
-// allocation does not change the arithmetic.
+// unbound (Brown+Neel Heun, 1024 particles: 1.70 us per step, 2.79 bound).  The
+// implicit-midpoint kernels are bound too (cubic Neel, 262144 particles, reference matrix:
+// 77 us per step, 89 with the 160 registers left alone; exact matrix: 28.5, 16 % faster than
+// unbound).  Register allocation does not change the arithmetic.
 //
 // Where the increments of a kernel with in-kernel noise are drawn (NOISE): inside the step,
 // where the pairs' chains interleave with the step's own (Cartesian problems, FP32 and the
@@ -337,7 +336,7 @@ template <int PROB, class R, int SOLVER, int NOISE, int PPT>
 constexpr int step_min_blocks() {
     return (sizeof(R) == 8 && NOISE != kCopied &&
             (SOLVER == kEulerMaruyama || SOLVER == kHeun || SOLVER == kMillstein || SOLVER == kEulerMaruyamaNormalized ||
-             SOLVER == kImplicitMidpointExact))
+             SOLVER == kImplicitMidpoint || SOLVER == kImplicitMidpointExact))
                ? 2
                : 0;
 }

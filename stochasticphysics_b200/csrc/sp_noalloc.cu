@@ -131,7 +131,7 @@ extern "C" SP_API sp_status sp_simulate_noalloc(const sp_ensemble_desc* desc, co
         e.seed = desc->seed; e.pid_offset = desc->particle_id_offset;
         e.dt = desc->timestep; e.sqrt_dt = std::sqrt(desc->timestep);
         e.field = field_params(desc->field);
-        e.max_iter = desc->max_iteration; e.tol = desc->accuracy_goal;
+        e.max_iter = desc->max_iteration; e.tol = R == 8 ? squared_tolerance(desc->accuracy_goal) : desc->accuracy_goal;
         e.dna = desc->double_noise_approx; e.rho = double_noise_rho(desc->double_noise_approx);
         const double kPi = 3.14159265358979323846;
         if (desc->problem == SP_PROBLEM_NEEL_SPHERICAL) {

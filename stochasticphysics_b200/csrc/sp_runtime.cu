@@ -53,6 +53,17 @@ double double_noise_rho(int p) {
     return std::sqrt(1.0 / 12.0 - s / (2.0 * kPi * kPi));
 }
 
+// the largest x with sqrt(x) <= tol: comparing x itself gives the same answer without the root
+double squared_tolerance(double tol) {
+    const double inf = std::numeric_limits<double>::infinity(), most = std::numeric_limits<double>::max();
+    if (!(tol > 0.0)) return tol;  // unused (validate_desc asks the implicit solver for > 0)
+    if (tol >= std::sqrt(most)) return std::isinf(tol) ? inf : most;
+    double x = tol * tol;
+    while (std::sqrt(x) > tol) x = std::nextafter(x, 0.0);
+    while (std::sqrt(std::nextafter(x, inf)) <= tol) x = std::nextafter(x, inf);
+    return x;
+}
+
 // ------------------------------------------------------------------ validation
 sp_status validate_desc(const sp_ensemble_desc* d, std::string& why) {
     auto bad = [&](const std::string& m) { why = m; return SP_ERR_INVALID_ARG; };
@@ -270,7 +281,7 @@ Ensemble::Ensemble(sp_context* c, const sp_ensemble_desc& d, const LaunchConfig&
     e.seed = d.seed; e.pid_offset = d.particle_id_offset;
     e.dt = d.timestep; e.sqrt_dt = std::sqrt(d.timestep);
     e.field = field_params(d.field);
-    e.max_iter = d.max_iteration; e.tol = d.accuracy_goal;
+    e.max_iter = d.max_iteration; e.tol = R == 8 ? squared_tolerance(d.accuracy_goal) : d.accuracy_goal;
     e.dna = d.double_noise_approx; e.rho = double_noise_rho(d.double_noise_approx);
     const double kPi = 3.14159265358979323846;
     if (d.problem == SP_PROBLEM_NEEL_SPHERICAL) {

@@ -98,7 +98,7 @@ struct EnsDev {
     int rot_brown;  // NeelSpherical: rotation enabled; BrownNeelEuler: Brown rotation enabled
     int rot_neel;   // BrownNeelEuler: Neel rotation enabled
     int slots;      // partial slots per chunk (max windows completing in a chunk)
-    double tol;
+    double tol;     // Newton acceptance: FP32 the tolerance; FP64 the largest square of it (squared_tolerance)
     double min1, max1, min2, max2;  // rotation thresholds
     // buffers
     void* state;

@@ -71,6 +71,12 @@ int main(int argc, char** argv) {
             for (int d = -2; d <= 2; ++d) for (int s = 0; s < 20; s += 5) one(((0x80000000u + (i << 23)) >> s) + (uint32_t)d);
     } else if (!strcmp(what, "sqrt")) {
         for (int i = 0; i < 300000; ++i) { const double x = ldexp(1 + unit(), (int)(g() % 120) - 90); see(sqrt_normal(x), sqrtq((Q)x)); }
+    } else if (!strcmp(what, "quotient")) {  // the correctly rounded quotient, bit for bit
+        for (int i = 0; i < 300000; ++i) {
+            const double b = (2 * unit() - 1) * ldexp(1, (int)(g() % 20) - 10), a = (2 * unit() - 1) * ldexp(1, (int)(g() % 80) - 70);
+            if (b != 0 && quotient(a, b, rcp_normal(b)) != a / b) worst = 1e9;
+        }
+        if (quotient(0.0, 3.0, rcp_normal(3.0)) != 0.0) worst = 1e9;
     } else {
         for (int i = 0; i < 300000; ++i) { const double x = (2 * unit() - 1) * ldexp(1, -(int)(g() % 60)); if (x != 0) see(rcp_or_zero(x), 1 / (Q)x); }
         if (rcp_or_zero(0.0) != 0.0 || rcp_or_zero(-0.0) != 0.0) worst = 1e9;
@@ -93,7 +99,7 @@ def program(tmp_path_factory):
 
 
 @pytest.mark.parametrize("what, bound", [("angle", 1.5), ("range", 1.5), ("turn", 1.5), ("log", 0.75), ("sqrt", 0.51),
-                                         ("reciprocal", 0.51)])
+                                         ("quotient", 0.0), ("reciprocal", 0.51)])
 def test_error_in_ulp(program, what, bound):
     worst = float(subprocess.run([str(program), what], check=True, capture_output=True, text=True).stdout)
     assert worst <= bound, f"{what}: {worst} ulp"
