@@ -259,19 +259,7 @@ Ensemble::Ensemble(sp_context* c, const sp_ensemble_desc& d, const LaunchConfig&
     // injected increments: [S][M][n] FP64 host -> [S][M][Np] Real device
     if (d.noise == SP_NOISE_INJECTED && L.S > 0) {
         d_dw = dalloc(L.S * L.Mn * L.Np * R);
-        const size_t rows = L.S * L.Mn;
-        std::vector<unsigned char> host(rows * L.Np * R, 0);
-        for (size_t r = 0; r < rows; ++r) {
-            const double* src = d.injected_dw + r * L.n;
-            if (R == 8) {
-                std::memcpy(host.data() + r * L.Np * 8, src, L.n * 8);
-            } else {
-                float* dst = reinterpret_cast<float*>(host.data() + r * L.Np * 4);
-                for (size_t i = 0; i < L.n; ++i) dst[i] = static_cast<float>(src[i]);
-            }
-        }
-        check_cuda(cudaMemcpyAsync(d_dw, host.data(), host.size(), cudaMemcpyHostToDevice, stream), "upload dW");
-        check_cuda(cudaStreamSynchronize(stream), "sync");
+        upload_increments(ctx, d.injected_dw, d_dw, L.real, L.S * L.Mn, L.n, L.Np, stream);
     }
 
     // device descriptor
@@ -700,6 +688,8 @@ sp_status sp_destroy(sp_context* ctx) {
         cudaMemPoolDestroy(ctx->pool);
     }
     if (ctx->stage) cudaFreeHost(ctx->stage);
+    for (double* p : ctx->dw_pinned)
+        if (p) cudaFreeHost(p);
     delete ctx;
     return SP_OK;
     SP_GUARD_END

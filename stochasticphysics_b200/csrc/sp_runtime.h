@@ -29,6 +29,10 @@ struct sp_context {
     std::mutex stage_mu;
     double* stage = nullptr;
     size_t stage_doubles = 0;
+    // pinned pieces of the injected increments' upload (sp_upload.cu, 16 MB at most), kept
+    // until the context is destroyed; nullptr where pinned memory could not be had
+    std::mutex dw_mu;
+    std::vector<double*> dw_pinned;
 };
 
 namespace sp {
@@ -50,6 +54,9 @@ int noise_dim(int p);
 int out_dim(int p);
 int param_count(int p, int aniso);
 double double_noise_rho(int p);
+// caller-supplied increments [rows][n] (host) -> [rows][Np] of `real` bytes each (sp_upload.cu)
+void upload_increments(sp_context* ctx, const double* src, void* dst, int real, size_t rows, size_t n, size_t Np,
+                       cudaStream_t s);
 double squared_tolerance(double tol);
 FieldParams field_params(const sp_field_desc& f);
 void reference_times(unsigned long long K, unsigned long long W, double dt, double* times);
