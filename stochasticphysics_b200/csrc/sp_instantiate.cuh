@@ -12,18 +12,18 @@ template <int PROB, class R, int A>
 size_t inj_smem_t(int threads) {
     return DwStream<R, ProblemOf<PROB, R, A>::type::Mn>::smem_bytes(threads);
 }
-template <int PROB, class R, int A>
+template <int PROB, class R, int A, int SOLVER>
 size_t drawn_smem_t(int threads) {
-    return DwStream<R, ProblemOf<PROB, R, A>::type::Mn>::smem_bytes_drawn(threads);
+    return static_cast<size_t>(threads / 32) * drawn_bytes_per_warp<typename StepProblem<PROB, R, A, SOLVER, kDrawn>::type>();
 }
 template <int PROB, class R, int A, int SOLVER, bool INJ>
 constexpr int noise_form() {
-    return INJ ? kCopied : (StepProblem<PROB, R, A, SOLVER>::type::kCarriedChart ? kDrawn : kInline);
+    return INJ ? kCopied : (StepProblem<PROB, R, A, SOLVER, kDrawn>::type::kCarriedChart ? kDrawn : kInline);
 }
 template <int PROB, class R, int A, int SOLVER, bool INJ, int PPT>
 void launch_step_t(const EnsDev* e, const TileDesc* t, int ntiles, int grid, int block, cudaStream_t s) {
     constexpr int F = noise_form<PROB, R, A, SOLVER, INJ>();
-    const size_t dyn = F == kCopied ? inj_smem_t<PROB, R, A>(block / PPT) : (F == kDrawn ? drawn_smem_t<PROB, R, A>(block / PPT) : 0);
+    const size_t dyn = F == kCopied ? inj_smem_t<PROB, R, A>(block / PPT) : (F == kDrawn ? drawn_smem_t<PROB, R, A, SOLVER>(block / PPT) : 0);
     step_kernel<PROB, R, A, SOLVER, F, PPT><<<grid, block / PPT, dyn, s>>>(e, t, ntiles);
 }
 // the injected kernels' staging exceeds the default dynamic shared memory limit: raise it
@@ -38,7 +38,7 @@ void prepare_ring_t() {
     if (done[dev]) return;
     if (cudaFuncSetAttribute(reinterpret_cast<const void*>(&step_kernel<PROB, R, A, SOLVER, F, 1>),
                              cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(F == kCopied ? inj_smem_t<PROB, R, A>(kMaxBlock) : drawn_smem_t<PROB, R, A>(kMaxBlock))) == cudaSuccess)
+                             static_cast<int>(F == kCopied ? inj_smem_t<PROB, R, A>(kMaxBlock) : drawn_smem_t<PROB, R, A, SOLVER>(kMaxBlock))) == cudaSuccess)
         done[dev] = true;
 }
 template <int PROB, class R, int A, int SOLVER>
@@ -84,7 +84,7 @@ KernelSet make_set() {
             k.prepare = &prepare_ring_t<PROB, R, A, SOLVER, kCopied>;
             if constexpr (sizeof(R) == 8) k.noise = &launch_noise_t<PROB, R, A, SOLVER>;
         } else if constexpr (noise_form<PROB, R, A, SOLVER, INJ>() == kDrawn) {
-            k.dyn_smem = &drawn_smem_t<PROB, R, A>;
+            k.dyn_smem = &drawn_smem_t<PROB, R, A, SOLVER>;
             k.prepare = &prepare_ring_t<PROB, R, A, SOLVER, kDrawn>;
         }
         k.reduce = &launch_reduce_t<Prob::OUT>;

@@ -33,11 +33,13 @@ template <class R, int A> struct ProblemOf<kNeelSpherical, R, A> { using type = 
 template <class R, int A> struct ProblemOf<kBrownNeelEuler, R, A> { using type = BrownNeelEuler<R, A>; static constexpr int P = param_count_of(kBrownNeelEuler, A); };
 template <class R, int A> struct ProblemOf<kBrownNeel, R, A> { using type = BrownNeelCart<R, A>; static constexpr int P = param_count_of(kBrownNeel, A); };
 // the form a solver's steps run in: sp_physics64.cuh's for the FP64 explicit steps of the angle problems
-template <int PROB, class R, int A, int SOLVER> struct StepProblem { using type = typename ProblemOf<PROB, R, A>::type; };
-template <int A, int SOLVER> struct StepProblem<kNeelSpherical, double, A, SOLVER> {
+template <int PROB, class R, int A, int SOLVER, int NOISE> struct StepProblem { using type = typename ProblemOf<PROB, R, A>::type; };
+template <int A, int SOLVER, int NOISE> struct StepProblem<kNeelSpherical, double, A, SOLVER, NOISE> {
     using type = std::conditional_t<SOLVER == kImplicitMidpoint, NeelSph<double, A>, NeelSphD<A>>;
 };
-template <int A, int SOLVER> struct StepProblem<kBrownNeelEuler, double, A, SOLVER> { using type = BrownNeelEulerD<A>; };
+template <int A, int SOLVER, int NOISE> struct StepProblem<kBrownNeelEuler, double, A, SOLVER, NOISE> {
+    using type = BrownNeelEulerD<A, NOISE == kDrawn && A != kUniaxialCubic>;
+};
 
 // ------------------------------------------------------------------ FP64 parameter formulas
 constexpr double kBoltzmann = 1.3806485279E-23;  // ParameterCalculatorNeel.h:43
@@ -249,6 +251,44 @@ struct WindowSum {
         }
     }
 };
+// FP64 sums kept in shared memory: (sum, compensation) of output c of this lane at
+// at + 512 c.  Volatile accesses, or the compiler keeps them in registers across the steps.
+template <int OUT>
+struct SharedWindowSum {
+    uint32_t at;
+    __device__ __forceinline__ void load(int c, double& s, double& k) const {
+        asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(s), "=d"(k) : "r"(at + 512u * static_cast<uint32_t>(c)));
+    }
+    __device__ __forceinline__ void set(int c, double s, double k) {
+        asm volatile("st.shared.v2.f64 [%0], {%1, %2};" ::"r"(at + 512u * static_cast<uint32_t>(c)), "d"(s), "d"(k));
+    }
+    __device__ __forceinline__ double get_sum(int c) const {
+        double s, k;
+        load(c, s, k);
+        return s;
+    }
+    __device__ __forceinline__ double get_comp(int c) const {
+        double s, k;
+        load(c, s, k);
+        return k;
+    }
+    __device__ __forceinline__ void clear_sum(int c) {
+        double s, k;
+        load(c, s, k);
+        set(c, 0.0, k);
+    }
+    __device__ __forceinline__ void add(const double* o) {
+        double s[OUT], k[OUT];
+#pragma unroll
+        for (int c = 0; c < OUT; ++c) load(c, s[c], k[c]);
+#pragma unroll
+        for (int c = 0; c < OUT; ++c) {
+            const double yv = o[c] - k[c];
+            const double tv = s[c] + yv;
+            set(c, tv, (tv - s[c]) - yv);
+        }
+    }
+};
 // FP32: two outputs per 64-bit register, both updated by one paired instruction
 // (add/sub.rn.f32x2); each lane rounds exactly as the scalar form does.
 __device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
@@ -331,7 +371,7 @@ struct WindowSum<float, OUT> {
 // Cartesian Heun, whose step is a third of that: 2.51 inside, 2.85 staged).
 // The angle problems' FP64 steps with the library's sines and pairs called one after another
 // and the chart rotated and turned back on every step: Brown+Neel Millstein, 65536 particles,
-// 9.17 us per step, now 4.10; Heun 12.4, now 5.96.
+// 9.17 us per step, now 3.76; Heun 12.4, now 5.49.
 template <int PROB, class R, int SOLVER, int NOISE, int PPT>
 constexpr int step_min_blocks() {
     return (sizeof(R) == 8 && NOISE != kCopied &&
@@ -340,10 +380,22 @@ constexpr int step_min_blocks() {
                ? 2
                : 0;
 }
+// prefactors a problem's steps keep in shared memory (SharedPar)
+template <class Prob, class = void> struct SharedPrefactors { static constexpr int n = 0; };
+template <class Prob> struct SharedPrefactors<Prob, std::void_t<decltype(Prob::kSharedPar)>> { static constexpr int n = Prob::kSharedPar; };
+template <class Prob> constexpr int shared_prefactors() { return SharedPrefactors<Prob>::n; }
+// dynamic shared memory of a warp that draws its increments: a stage, then the prefactors and
+// window sums kept there
+template <class Prob>
+constexpr size_t drawn_bytes_per_warp() {
+    return DwStream<double, Prob::Mn, true>::kStageBytes +
+           (shared_prefactors<Prob>() ? 256u * shared_prefactors<Prob>() + 512u * Prob::OUT : 0u);
+}
 template <int PROB, class R, int A, int SOLVER, int NOISE, int PPT>
 __global__ void __launch_bounds__(kMaxBlock / PPT, (step_min_blocks<PROB, R, SOLVER, NOISE, PPT>()))
     step_kernel(const EnsDev* __restrict__ ensembles, const TileDesc* __restrict__ tiles, int ntiles) {
-    using Prob = typename StepProblem<PROB, R, A, SOLVER>::type;
+    using Prob = typename StepProblem<PROB, R, A, SOLVER, NOISE>::type;
+    constexpr int kSharedPar = shared_prefactors<Prob>();
     using St = Stepper<Prob, R, SOLVER>;
     constexpr int D = Prob::D, Mn = Prob::Mn, OUT = Prob::OUT;
     // per-warp copy of the chunk's field table: warps never wait on each other
@@ -357,11 +409,12 @@ __global__ void __launch_bounds__(kMaxBlock / PPT, (step_min_blocks<PROB, R, SOL
     __shared__ ChartBounds sCharts[Prob::kCarriedChart ? kMaxBlock / 32 : 1][2];
     ChartBounds* const charts = sCharts[Prob::kCarriedChart ? threadIdx.x >> 5 : 0];
     // each warp's ring of increments, copied or drawn (dynamic shared memory)
-    using Stream = DwStream<R, Mn>;
+    using Stream = DwStream<R, Mn, NOISE == kDrawn>;
     constexpr bool kLibraryNoise = SOLVER == kImplicitMidpoint || SOLVER == kImplicitMidpointExact;
     if constexpr (NOISE != kCopied) load_noise_tables<R>();
     static_assert(!kRing || PPT == 1, "injected increments are staged for one particle per thread");
     Stream dws;
+    [[maybe_unused]] uint32_t shared_at = 0;  // after a drawn stage: the warp's prefactors and window sums
     if constexpr (kRing) {
         extern __shared__ __align__(128) unsigned char sp_dyn_smem[];
         __shared__ uint64_t sbar[kMaxBlock / 32][Stream::kStages];
@@ -369,7 +422,9 @@ __global__ void __launch_bounds__(kMaxBlock / PPT, (step_min_blocks<PROB, R, SOL
         // the launch sizes the ring: kStages stages per warp (copied increments) or one (drawn)
         uint32_t dyn;
         asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn));
-        dws.init(reinterpret_cast<R*>(sp_dyn_smem + static_cast<size_t>(warp) * (dyn / (blockDim.x >> 5))), sbar[warp]);
+        unsigned char* const mine = sp_dyn_smem + static_cast<size_t>(warp) * (dyn / (blockDim.x >> 5));
+        dws.init(reinterpret_cast<R*>(mine), sbar[warp]);
+        shared_at = smem_addr(mine) + Stream::kStageBytes;
     }
 
     for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
@@ -399,7 +454,7 @@ __global__ void __launch_bounds__(kMaxBlock / PPT, (step_min_blocks<PROB, R, SOL
 
         R y[PPT][D];
         R lo[PPT][D];  // FP32 form: the carried rounding errors of the slowly moving components
-        WindowSum<R, OUT> acc[PPT];
+        std::conditional_t<(kSharedPar > 0), SharedWindowSum<OUT>, WindowSum<R, OUT>> acc[PPT];
         typename Prob::Par q[PPT];
         typename Prob::Trig tr[PPT];  // sincos of y, carried from each step's output to the next prepare
         if constexpr (Prob::kCarriedChart) {
@@ -412,6 +467,14 @@ __global__ void __launch_bounds__(kMaxBlock / PPT, (step_min_blocks<PROB, R, SOL
         }
 #pragma unroll
         for (int k = 0; k < PPT; ++k) {
+            if constexpr (kSharedPar > 0) {
+                const uint32_t lane = threadIdx.x & 31;
+                acc[k].at = shared_at + 256u * kSharedPar + 16u * lane;
+                q[k].at = shared_at + 8u * lane;
+                const unsigned long long pp = active[k] ? p[k] : td.first;
+                for (int i = 0; i < kSharedPar; ++i)
+                    asm volatile("st.shared.f64 [%0], %1;" ::"r"(q[k].at + 256u * i), "d"(static_cast<const double*>(e.params)[i * Np + pp]));
+            }
             if (active[k]) {
                 const R* state = static_cast<const R*>(e.state);
                 const R* ks = static_cast<const R*>(e.ksum);
@@ -420,13 +483,13 @@ __global__ void __launch_bounds__(kMaxBlock / PPT, (step_min_blocks<PROB, R, SOL
                 for (int i = 0; i < D; ++i) y[k][i] = state[i * Np + p[k]];
 #pragma unroll
                 for (int c = 0; c < OUT; ++c) acc[k].set(c, ks[c * Np + p[k]], kc[c * Np + p[k]]);
-                q[k] = Prob::load(static_cast<const R*>(e.params), Np, p[k]);
+                if constexpr (kSharedPar == 0) q[k] = Prob::load(static_cast<const R*>(e.params), Np, p[k]);
             } else {
 #pragma unroll
                 for (int i = 0; i < D; ++i) y[k][i] = R(0);
 #pragma unroll
                 for (int c = 0; c < OUT; ++c) acc[k].set(c, R(0), R(0));
-                q[k] = Prob::load(static_cast<const R*>(e.params), Np, td.first);  // any valid slot; results are discarded
+                if constexpr (kSharedPar == 0) q[k] = Prob::load(static_cast<const R*>(e.params), Np, td.first);  // any valid slot; results are discarded
             }
             Prob::trig(y[k], tr[k]);
             if constexpr (Prob::kCarriedChart) {
@@ -534,7 +597,7 @@ __global__ void __launch_bounds__(kMaxBlock / PPT, (step_min_blocks<PROB, R, SOL
                 };
                 for (int i = 0; i < len; ++i) {
                     R cur[PPT][Mn];
-                    if (!dws.template next<NOISE == kDrawn>(cur[0], draw)) break;  // a stage timed out (uniform across the warp)
+                    if (!dws.next(cur[0], draw)) break;  // a stage timed out (uniform across the warp)
                     one_step(i, cur);
                 }
                 if (!dws.ok) break;

@@ -14,6 +14,8 @@
 // Brown+Neel, FP64 (B200, one ensemble at a time): see step_min_blocks in sp_kernels.cuh.
 #pragma once
 
+#include <type_traits>
+
 #include "sp_physics.cuh"
 
 namespace sp {
@@ -198,12 +200,37 @@ struct NeelSphD : NeelSph<double, A> {
 };
 
 // ======================================================================= Brown + Neel, Euler/spherical
-template <int A>
+// SHARED: the prefactors and the window sums live in shared memory, one column per lane, and
+// are read where a formula uses them: 13 prefactors and 9 sums with their compensations are
+// 62 of the 128 registers a thread has, and the compiler spilled 600-800 bytes of them and of
+// the step's temporaries to local memory (now 100-200).  65536 particles, Millstein / Heun: 4.06 /
+// 5.96 us per step in registers, 3.76 / 5.49 shared; 262144: 12.9 / - and 11.9 / -.  Not for
+// the uniaxial+cubic anisotropy, whose 24 prefactors leave no room for a second CTA, nor where
+// the increments are copied: those run few warps, unbound in registers.
+struct SharedPar {
+    uint32_t at;  // shared address of the lane's prefactor 0; prefactor i is 256 i bytes on
+};
+template <int A, bool SHARED = false>
 struct BrownNeelEulerD : BrownNeelEuler<double, A> {
     using Base = BrownNeelEuler<double, A>;
-    using Par = typename Base::Par;
+    using Par = std::conditional_t<SHARED, SharedPar, typename Base::Par>;
     using Cache = typename Base::Cache;
     static constexpr bool kCarriedChart = true;
+    static constexpr int kSharedPar = SHARED ? kParamsBrownNeelEuler : 0;
+    // the prefactors in registers; unused ones are not read
+    static __device__ __forceinline__ typename Base::Par params(const Par& q) {
+        if constexpr (SHARED) {
+            uint32_t at = q.at;
+            asm volatile("" : "+r"(at));  // read again, not kept from an earlier use
+            return Base::load_with([&](int i) {
+                double v;
+                asm("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(at + 256u * static_cast<uint32_t>(i)));
+                return v;
+            });
+        } else {
+            return q;
+        }
+    }
     // sines and cosines of the state's angles, which are those of the charts br, nr
     struct Trig {
         double S[5], C[5];
@@ -253,7 +280,8 @@ struct BrownNeelEulerD : BrownNeelEuler<double, A> {
     }
     static __device__ __forceinline__ void finish(const Rot<double>&, double* y, const Cache&) { wrap_angles<5>(y); }
     // :363-425
-    static __device__ __forceinline__ void det(const Par& q, const double*, const Cache& c, const double* B, double* a) {
+    static __device__ __forceinline__ void det(const Par& par, const double*, const Cache& c, const double* B, double* a) {
+        const typename Base::Par q = params(par);
         V3<double> x, y, z;
         axes(c.S, c.C, c.br, x, y, z);
         const V3<double> H = Base::heff(q, c.md, x, y, z, B);
@@ -264,7 +292,8 @@ struct BrownNeelEulerD : BrownNeelEuler<double, A> {
         sproj(c, (-q.a) * H + q.bpd * mxH + cTe, a + 3);
     }
     // :427-497 applied to w = (wA, wB)
-    static __device__ __forceinline__ void bdw(const Par& q, const double*, const Cache& c, const double* w, double* r) {
+    static __device__ __forceinline__ void bdw(const Par& par, const double*, const Cache& c, const double* w, double* r) {
+        const typename Base::Par q = params(par);
         const V3<double> wA = v3(w[0], w[1], w[2]), wB = v3(w[3], w[4], w[5]);
         const V3<double> cwA = q.cF * wA;
         const V3<double> mxw = cross(c.md, wB);  // shared by both rows
@@ -273,7 +302,8 @@ struct BrownNeelEulerD : BrownNeelEuler<double, A> {
         sproj(c, cwA + q.bpdDN * mxw - q.aDN * wB, r + 3);
     }
     // :499-601: both charts alike by straight-line code, else (rare) replaced
-    static __device__ __forceinline__ void drift(const Par& q, const double*, const Cache& c, double* r) {
+    static __device__ __forceinline__ void drift(const Par& par, const double*, const Cache& c, double* r) {
+        const typename Base::Par q = params(par);
         const double ctheta = c.C[1], cpsi = c.C[2], spsi = c.S[2];
         const double cos_t = c.C[3], cos_p = c.C[4], sin_t = c.S[3], sin_p = c.S[4];
         const double csc = c.csc;

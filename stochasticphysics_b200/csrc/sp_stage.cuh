@@ -58,13 +58,14 @@ __device__ __forceinline__ void bulk_copy_g2s(uint32_t dst, const void* src, uin
                  : "memory");
 }
 
-// Kernels that draw their noise a stage at a time use the same buffer, one stage, each lane
-// writing and reading its own column.
+// Kernels that draw their noise a stage at a time (DRAWN) use the same buffer, one stage, each
+// lane writing and reading its own column; two steps of six increments or four of three, 3 KB
+// per warp either way.
 
 // The increments of one warp's 32 particles for the steps of one tile, in order.
-template <class R, int Mn>
+template <class R, int Mn, bool DRAWN = false>
 struct DwStream {
-    static constexpr int kStep = 4;    // steps per stage
+    static constexpr int kStep = DRAWN && Mn > 3 ? 2 : 4;  // steps per stage
     static constexpr int kStages = 3;  // stages in the ring
     static constexpr int kRow = 32 * static_cast<int>(sizeof(R));
     static constexpr int kStageBytes = kStep * Mn * kRow;
@@ -73,8 +74,6 @@ struct DwStream {
 
     // dynamic shared memory of a CTA of `threads` threads
     static constexpr size_t smem_bytes(int threads) { return static_cast<size_t>(threads / 32) * kStages * kStageBytes; }
-    // drawn in the kernel: one stage per warp
-    static constexpr size_t smem_bytes_drawn(int threads) { return static_cast<size_t>(threads / 32) * kStageBytes; }
 
     R* buf;               // this warp's ring: [kStages][kStep][Mn][32]
     uint32_t bar0;        // its first barrier (8 bytes apart)
@@ -142,7 +141,7 @@ struct DwStream {
     // timed out (uniform across the warp)
     // draw(first, j, steps): writes the increments of steps j .. j + steps - 1 of the tile to
     // first[(s Mn + m) 32]
-    template <bool DRAWN, class Draw>
+    template <class Draw>
     __device__ __forceinline__ bool next(R* w, Draw draw) {
         const int within = static_cast<int>(pos % kStep);
         if constexpr (DRAWN) {  // this lane's own draws, the whole stage at once
