@@ -152,6 +152,22 @@ LaunchConfig default_launch(const sp_context* ctx, const sp_ensemble_desc& d) {
     int block = 256;
     const unsigned long long n = d.n_particles;
     while (block > 32 && (n + block - 1) / block < static_cast<unsigned long long>(2 * sms)) block >>= 1;
+    // One residency is 16 warps per SM at 128 registers, four per scheduler.
+    const unsigned long long warp_per_sm = 32ull * static_cast<unsigned long long>(sms);
+    if (d.precision == SP_PRECISION_FP64) {
+        // Four warps on some scheduler whatever the tile: the largest one, whose warps share
+        // their instruction fetches (66000 particles, 256 / 128 threads, us per step: Neel Heun
+        // 1.41 / 1.48, Neel spherical Euler-Maruyama 1.81 / 1.86, Brown+Neel Heun 5.51 / 5.70,
+        // cubic implicit 23.1 / 24.1).  Below 12 warps per SM a smaller tile spreads evener
+        // (50000: Neel Heun 1.41 / 1.15).
+        if (n > 12 * warp_per_sm) block = 256;
+    } else if (d.problem == SP_PROBLEM_BROWN_AND_NEEL_EULER_SPHERICAL && n > 16 * warp_per_sm) {
+        // More than one residency, and warps of unequal length (chart rotations diverge): small
+        // tiles free their slots sooner (FP32 Heun, 262144 particles: 256 threads 10.04 us per
+        // step, 128 9.27, 64 9.24; Millstein, 131072: 4.66, 4.13, 3.98).  The other problems
+        // move by 2 % or less.
+        block = 64;
+    }
     c.block = block;
     c.persistent = 0;
     const unsigned long long W = d.oversampling;
@@ -203,15 +219,23 @@ void* Ensemble::dalloc(size_t bytes) {
 // warps per SM scheduler, an FP64 ensemble with in-kernel noise therefore draws each chunk's
 // increments in a separate, fully parallel kernel (the same Philox counters and
 // arithmetic, so the results are bit-identical) into a chunk-sized buffer that the
-// injected step kernel stages like caller-supplied increments.  At 37888 particles, the
-// limit, Brown+Neel Heun / Millstein take 3.33 / 2.39 us per step against 3.77 / 2.54 drawn
-// in the kernel, Neel Heun 1.03 against 0.83.
-constexpr unsigned long long kPregenWarpsPerSM = 8;  // measured crossover: between 7 and 10
+// injected step kernel stages like caller-supplied increments.
+//
+// Up to how many particles per SM the separate draw wins (measured, us per step drawn before /
+// in the step): Brown+Neel Euler/spherical to the two warps per scheduler its unbound kernel
+// can have (37888 particles, Heun 3.27 / 3.77), the implicit steps alike; Neel Heun 20001
+// particles 0.77 / 0.82, 30011 0.91 / 0.83; Neel spherical Euler-Maruyama 20001 1.05 / 1.13, 30011
+// 1.24 / 1.17; Brown+Neel Cartesian Heun, whose six draws hide behind its own step, 4096
+// particles 0.78 / 0.87, 9000 0.90 / 0.87.
 constexpr unsigned long long kPregenBytes = 256ull << 20;  // cap on the chunk's increments buffer
+static unsigned long long pregen_particles_per_sm(const sp_ensemble_desc& d) {
+    if (d.solver == SP_SOLVER_IMPLICIT_MIDPOINT || d.problem == SP_PROBLEM_BROWN_AND_NEEL_EULER_SPHERICAL) return 8 * 32;
+    return d.problem == SP_PROBLEM_BROWN_AND_NEEL ? 3 * 16 : 5 * 32;
+}
 
 static bool pregen_wanted(const sp_context* ctx, const sp_ensemble_desc& d) {
     if (d.noise != SP_NOISE_PHILOX || d.precision != SP_PRECISION_FP64) return false;
-    if (d.n_particles > kPregenWarpsPerSM * 32ull * static_cast<unsigned long long>(ctx->sms)) return false;
+    if (d.n_particles > pregen_particles_per_sm(d) * static_cast<unsigned long long>(ctx->sms)) return false;
     const KernelSet& inj = kernel_set(d.problem, d.anisotropy, solver_slot(d.solver, d.jacobian), d.precision, 1);
     return inj.valid && inj.noise;
 }
