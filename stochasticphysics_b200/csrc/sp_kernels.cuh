@@ -434,7 +434,11 @@ __global__ void __launch_bounds__(kMaxBlock / PPT, (step_min_blocks<PROB, R, SOL
         const unsigned long long nsteps = tgt > s0 ? min(e.chunk, tgt - s0) : 0ull;
         if (nsteps == 0) continue;  // uniform across the CTA
         const unsigned long long Np = e.Np, W = e.W;
-        unsigned long long p[PPT];
+        // Lanes past the ensemble's end run the last particle's steps and store nothing, which
+        // saves a branch around each step (kSkipIdle: kept where it costs registers instead).
+        if (td.first + (threadIdx.x & ~31u) >= e.n) continue;  // a warp with none; no CTA barrier in this loop
+        constexpr bool kSkipIdle = NOISE == kDrawn;
+        unsigned long long p[PPT], pe[PPT];
         bool active[PPT];
         // A load through e inside the step loop is repeated every step (the window stores might
         // alias it).  The Cartesian problems keep the offset (FP32 Neel Heun, 65536 particles:
@@ -446,6 +450,7 @@ __global__ void __launch_bounds__(kMaxBlock / PPT, (step_min_blocks<PROB, R, SOL
         for (int k = 0; k < PPT; ++k) {
             p[k] = td.first + static_cast<unsigned long long>(k) * blockDim.x + threadIdx.x;
             active[k] = p[k] < e.n;
+            pe[k] = active[k] ? p[k] : e.n - 1;
         }
         const double dt_d = e.dt;
         const R dt = static_cast<R>(dt_d);
@@ -477,34 +482,27 @@ __global__ void __launch_bounds__(kMaxBlock / PPT, (step_min_blocks<PROB, R, SOL
                 const uint32_t lane = threadIdx.x & 31;
                 acc[k].at = shared_at + 256u * kSharedPar + 16u * lane;
                 q[k].at = shared_at + 8u * lane;
-                const unsigned long long pp = active[k] ? p[k] : td.first;
                 for (int i = 0; i < kSharedPar; ++i)
-                    asm volatile("st.shared.f64 [%0], %1;" ::"r"(q[k].at + 256u * i), "d"(static_cast<const double*>(e.params)[i * Np + pp]));
+                    asm volatile("st.shared.f64 [%0], %1;" ::"r"(q[k].at + 256u * i), "d"(static_cast<const double*>(e.params)[i * Np + pe[k]]));
             }
-            if (active[k]) {
+            {
                 const R* state = static_cast<const R*>(e.state);
                 const R* ks = static_cast<const R*>(e.ksum);
                 const R* kc = static_cast<const R*>(e.kcomp);
 #pragma unroll
-                for (int i = 0; i < D; ++i) y[k][i] = state[i * Np + p[k]];
+                for (int i = 0; i < D; ++i) y[k][i] = state[i * Np + pe[k]];
 #pragma unroll
-                for (int c = 0; c < OUT; ++c) acc[k].set(c, ks[c * Np + p[k]], kc[c * Np + p[k]]);
-                if constexpr (kSharedPar == 0) q[k] = Prob::load(static_cast<const R*>(e.params), Np, p[k]);
-            } else {
-#pragma unroll
-                for (int i = 0; i < D; ++i) y[k][i] = R(0);
-#pragma unroll
-                for (int c = 0; c < OUT; ++c) acc[k].set(c, R(0), R(0));
-                if constexpr (kSharedPar == 0) q[k] = Prob::load(static_cast<const R*>(e.params), Np, td.first);  // any valid slot; results are discarded
+                for (int c = 0; c < OUT; ++c) acc[k].set(c, ks[c * Np + pe[k]], kc[c * Np + pe[k]]);
+                if constexpr (kSharedPar == 0) q[k] = Prob::load(static_cast<const R*>(e.params), Np, pe[k]);
             }
             Prob::trig(y[k], tr[k]);
             if constexpr (Prob::kCarriedChart) {
-                Prob::set_chart(active[k] ? e.status[p[k]] : 0, tr[k]);
+                Prob::set_chart(e.status[pe[k]], tr[k]);
                 if (s0 == 0) Prob::rechart(charts, y[k], tr[k]);
             }
             const R* slo = static_cast<const R*>(e.slo);
 #pragma unroll
-            for (int i = 0; i < D; ++i) lo[k][i] = (slo && active[k]) ? slo[i * Np + p[k]] : R(0);
+            for (int i = 0; i < D; ++i) lo[k][i] = slo ? slo[i * Np + pe[k]] : R(0);
         }
         NewtonCount nc{0u, 0u};
         // W < 2^31 (validated); the window position fits 32 bits.  Values used only
@@ -512,6 +510,10 @@ __global__ void __launch_bounds__(kMaxBlock / PPT, (step_min_blocks<PROB, R, SOL
         // live in registers across the step loop.
         unsigned int wpos = static_cast<unsigned int>(s0 % W);
         const unsigned int W32 = static_cast<unsigned int>(W);
+        // the lane whose ring column this lane reads: its own, or the last particle's
+        [[maybe_unused]] const int column = static_cast<int>(
+            NOISE == kCopied ? min(static_cast<unsigned long long>(threadIdx.x & 31u), e.n - 1 - (td.first + (threadIdx.x & ~31u)))
+                             : threadIdx.x & 31u);
         // copied increments stream from HBM: the warp's rows of the tile's first steps go
         // in flight now (the warp's 32 particles start at the tile's first + 32 warp)
         if constexpr (kRing)
@@ -522,18 +524,17 @@ __global__ void __launch_bounds__(kMaxBlock / PPT, (step_min_blocks<PROB, R, SOL
             __syncwarp();
             for (int i = threadIdx.x & 31; i < 3 * len; i += 32) (&sB[0][0])[i] = ftab[3 * t0 + i];
             __syncwarp();
-            // one step of every particle of the thread; winj: the injected increments
-            auto one_step = [&](int i, const R (*winj)[Mn]) {
+            // one step of every particle of the thread in the field B; winj: the ring's increments
+            auto one_step = [&](int i, const R* B, const R* winj) {
                 const unsigned long long g = s0 + t0 + i;
-                const R B[3] = {sB[i][0], sB[i][1], sB[i][2]};
 #pragma unroll
                 for (int k = 0; k < PPT; ++k) {
-                    if (!active[k]) continue;
-                    const unsigned long long pid = (kKeepOffset ? kept_offset : e.pid_offset) + p[k];
+                    if (kSkipIdle && !active[k]) continue;
+                    [[maybe_unused]] const unsigned long long pid = (kKeepOffset ? kept_offset : e.pid_offset) + p[k];
                     R w[Mn];
                     if constexpr (kRing) {
 #pragma unroll
-                        for (int j = 0; j < Mn; ++j) w[j] = winj[k][j];
+                        for (int j = 0; j < Mn; ++j) w[j] = winj[j];
                     } else {
                         if constexpr (kLibraryNoise && sizeof(R) == 8) philox_increments_any<Mn>(seed, pid, g, sqdt, w);
                         else philox_increments<R, Mn>(seed, pid, g, m2dt, w);
@@ -550,17 +551,20 @@ __global__ void __launch_bounds__(kMaxBlock / PPT, (step_min_blocks<PROB, R, SOL
                         if constexpr (SOLVER == kWeakTest) St::step_weak(q[k], rot, y[k], B, w, An, dt, sqdt, tr[k]);
                         else St::step_es1(q[k], rot, y[k], B, w, An, dt, sqdt, tr[k]);
                     } else {
+                        const NewtonCount before = nc;
                         St::step(q[k], rot, y[k], B, w, dt, e.max_iter, e.tol, nc, tr[k],
                                  M<R>::kCompensatedState ? lo[k] : nullptr);
+                        if (!active[k]) nc = before;
                     }
                     R o[OUT];
                     Prob::out_t(y[k], o, tr[k]);
                     if constexpr (Prob::kCarriedChart) Prob::rechart(charts, y[k], tr[k]);
                     acc[k].add(o);
                 }
-                if (++wpos == W32) {  // window end: uniform across the CTA
-                    wpos = 0;
-                    const unsigned long long kw = (g + 1) / W;
+            };
+            // the window that ends with the first `done` steps of the run; uniform across the CTA
+            auto window_end = [&](unsigned long long done) {
+                    const unsigned long long kw = done / W;
                     const int slot = static_cast<int>(kw - s0 / W - 1);
                     double* const traj = e.traj;
 #pragma unroll
@@ -585,31 +589,59 @@ __global__ void __launch_bounds__(kMaxBlock / PPT, (step_min_blocks<PROB, R, SOL
                         }
                         if (lane < OUT) partial[lane] = mine;
                     }
+            };
+            // in-kernel noise (FP64): a stage of steps is drawn at a time, a small loop of its
+            // own whose independent pairs interleave, instead of inside the step's chain
+            [[maybe_unused]] auto draw = [&](R* first, unsigned long long j, int steps) {
+                if constexpr (NOISE == kDrawn) {
+                    const unsigned long long pid = e.pid_offset + p[0];
+                    for (int st = 0; st < steps; ++st) {
+                        R w[Mn];
+                        philox_increments<R, Mn>(seed, pid, s0 + j + st, m2dt, w);
+#pragma unroll
+                        for (int m = 0; m < Mn; ++m) first[(st * Mn + m) * 32] = w[m];
+                    }
                 }
             };
-            if constexpr (kRing) {
-                // in-kernel noise (FP64): a stage of steps is drawn at a time, a small loop of its
-                // own whose independent pairs interleave, instead of inside the step's chain
-                auto draw = [&](R* first, unsigned long long j, int steps) {
-                    if constexpr (NOISE == kDrawn) {
-                        const unsigned long long pid = e.pid_offset + p[0];
-                        for (int st = 0; st < steps; ++st) {
-                            R w[Mn];
-                            philox_increments<R, Mn>(seed, pid, s0 + j + st, m2dt, w);
-#pragma unroll
-                            for (int m = 0; m < Mn; ++m) first[(st * Mn + m) * 32] = w[m];
-                        }
-                    }
-                };
-                for (int i = 0; i < len; ++i) {
-                    R cur[PPT][Mn];
-                    if (!dws.next(cur[0], draw)) break;  // a stage timed out (uniform across the warp)
-                    one_step(i, cur);
+            // Runs of steps without a window end or a new stage inside them, so that a step is one
+            // basic block (a branch stops the scheduler from filling the FP64 chains' gaps with the
+            // next step's work): Neel Heun, 1024 particles, 0.428 us per step with the checks and an
+            // idle-lane branch inside, 0.391 in runs of at most four steps, 0.353 of eight; Neel
+            // spherical Euler-Maruyama 0.737, 0.621, 0.579.  Not where a step is long and the
+            // registers are all taken (Brown+Neel Euler drawing its noise: 3.68 us checked, 3.77
+            // in runs).
+            constexpr bool kRuns = NOISE == kCopied || (NOISE == kInline && PROB != kBrownNeelEuler);
+            for (int i = 0; i < len;) {
+                int run = kRuns ? static_cast<int>(min(static_cast<unsigned int>(len - i), W32 - wpos)) : 1;
+                [[maybe_unused]] const R* rows = nullptr;
+                if constexpr (kRing) {
+                    if (!dws.ready(draw)) break;  // a stage timed out (uniform across the warp)
+                    if constexpr (kRuns) run = min(run, dws.left());
+                    rows = dws.rows() + column;
                 }
-                if (!dws.ok) break;
-            } else {
-                for (int i = 0; i < len; ++i) one_step(i, nullptr);
+                // a Neel step is short enough for four to be scheduled as one (1024 particles,
+                // Heun: 0.353 us per step one at a time, 0.342 by fours; longer steps gain nothing)
+                constexpr int kUnroll = NOISE == kCopied && PROB == kNeel && SOLVER != kImplicitMidpoint && SOLVER != kImplicitMidpointExact ? 4 : 1;
+#pragma unroll kUnroll
+                for (int j = 0; j < run; ++j) {
+                    const R B[3] = {sB[i + j][0], sB[i + j][1], sB[i + j][2]};
+                    R w[kRing ? Mn : 1];
+                    if constexpr (kRing) {
+#pragma unroll
+                        for (int m = 0; m < Mn; ++m) w[m] = rows[(j * Mn + m) * 32];
+                    }
+                    one_step(i + j, B, w);
+                }
+                if constexpr (kRing) dws.used(run);
+                i += run;
+                wpos += static_cast<unsigned int>(run);
+                if (wpos == W32) {
+                    wpos = 0;
+                    window_end(s0 + t0 + i);
+                }
             }
+            if constexpr (kRing)
+                if (!dws.ok) break;
         }
         if constexpr (kRing) {
             if (!dws.ok) {  // report, wait for the copies still in flight, leave the results unwritten
