@@ -37,12 +37,10 @@ template <class R>
 struct SphRot {
     R t, p, st, ct, sp, cp;
 };
-// NeelRelaxationSpherical.h:568-602 (INV: the inverse rotation)
+// NeelRelaxationSpherical.h:568-602 (INV: the inverse rotation), from the angles' sines and
+// cosines
 template <class R, bool INV>
-__device__ __forceinline__ SphRot<R> sph_rotate_impl(R t0, R p0) {
-    R st, ct, sp, cp;
-    M<R>::sincos(t0, &st, &ct);
-    M<R>::sincos(p0, &sp, &cp);
+__device__ __forceinline__ SphRot<R> sph_rotate_from(R st, R ct, R sp, R cp) {
     SphRot<R> r;
     if constexpr (!INV) {
         r.t = M<R>::acos(-cp * st); r.p = M<R>::atan2(sp * st, ct);
@@ -52,6 +50,13 @@ __device__ __forceinline__ SphRot<R> sph_rotate_impl(R t0, R p0) {
     M<R>::sincos(r.t, &r.st, &r.ct);
     M<R>::sincos(r.p, &r.sp, &r.cp);
     return r;
+}
+template <class R, bool INV>
+__device__ __forceinline__ SphRot<R> sph_rotate_impl(R t0, R p0) {
+    R st, ct, sp, cp;
+    M<R>::sincos(t0, &st, &ct);
+    M<R>::sincos(p0, &sp, &cp);
+    return sph_rotate_from<R, INV>(st, ct, sp, cp);
 }
 template <class R, bool INV>
 __device__ __noinline__ SphRot<R> sph_rotate_cold(R t0, R p0) { return sph_rotate_impl<R, INV>(t0, p0); }
@@ -64,11 +69,10 @@ template <class R>
 struct EulerRot {
     R e0, e1, e2, s0, s1, s2, c0, c1, c2;
 };
-// BrownAndNeelRelaxationEulerSpherical.h:859-899 (INV: the inverse rotation)
+// BrownAndNeelRelaxationEulerSpherical.h:859-899 (INV: the inverse rotation), from the angles'
+// sines and cosines
 template <class R, bool INV>
-__device__ __forceinline__ EulerRot<R> euler_rotate_impl(R a0, R a1, R a2) {
-    R S0, C0, S1, C1, S2, C2;
-    M<R>::sincos(a0, &S0, &C0); M<R>::sincos(a1, &S1, &C1); M<R>::sincos(a2, &S2, &C2);
+__device__ __forceinline__ EulerRot<R> euler_rotate_from(R S0, R C0, R S1, R C1, R S2, R C2) {
     EulerRot<R> r;
     if constexpr (!INV) {
         r.e0 = M<R>::atan2(-C2 * C0 + C1 * S0 * S2, S0 * C2 + C1 * C0 * S2);
@@ -81,6 +85,12 @@ __device__ __forceinline__ EulerRot<R> euler_rotate_impl(R a0, R a1, R a2) {
     }
     M<R>::sincos(r.e0, &r.s0, &r.c0); M<R>::sincos(r.e1, &r.s1, &r.c1); M<R>::sincos(r.e2, &r.s2, &r.c2);
     return r;
+}
+template <class R, bool INV>
+__device__ __forceinline__ EulerRot<R> euler_rotate_impl(R a0, R a1, R a2) {
+    R S0, C0, S1, C1, S2, C2;
+    M<R>::sincos(a0, &S0, &C0); M<R>::sincos(a1, &S1, &C1); M<R>::sincos(a2, &S2, &C2);
+    return euler_rotate_from<R, INV>(S0, C0, S1, C1, S2, C2);
 }
 template <class R, bool INV>
 __device__ __noinline__ EulerRot<R> euler_rotate_cold(R a0, R a1, R a2) { return euler_rotate_impl<R, INV>(a0, a1, a2); }
@@ -370,7 +380,7 @@ struct NeelSph {
     static __device__ __forceinline__ void prepare_t(const Par& q, const Rot<R>& r, R* y, Cache& c, const Trig& t) {
         c.rot = r.rb && (y[0] < r.min1 || y[0] > r.max1);
         if (c.rot) {
-            const SphRot<R> n = sph_rotate<R, false>(y[0], y[1]);
+            const SphRot<R> n = sph_rotate_from<R, false>(t.st, t.ct, t.sp, t.cp);
             y[0] = n.t; y[1] = n.p;
             cache_from(q, n.st, n.ct, n.sp, n.cp, c);
         } else {
@@ -600,7 +610,7 @@ struct BrownNeelEuler {
     static __device__ __forceinline__ void prepare_flags(const Par&, R* y, Cache& c, const Trig& t, bool br, bool nr) {
         c.br = br;
         if (c.br) {
-            const EulerRot<R> n = sp::euler_rotate<R, false>(y[0], y[1], y[2]);
+            const EulerRot<R> n = euler_rotate_from<R, false>(t.S[0], t.C[0], t.S[1], t.C[1], t.S[2], t.C[2]);
             y[0] = n.e0; y[1] = n.e1; y[2] = n.e2;
             c.S[0] = n.s0; c.S[1] = n.s1; c.S[2] = n.s2; c.C[0] = n.c0; c.C[1] = n.c1; c.C[2] = n.c2;
         } else {
@@ -609,7 +619,7 @@ struct BrownNeelEuler {
         }
         c.nr = nr;
         if (c.nr) {
-            const SphRot<R> n = sph_rotate<R, false>(y[3], y[4]);
+            const SphRot<R> n = sph_rotate_from<R, false>(t.S[3], t.C[3], t.S[4], t.C[4]);
             y[3] = n.t; y[4] = n.p;
             c.S[3] = n.st; c.C[3] = n.ct; c.S[4] = n.sp; c.C[4] = n.cp;
         } else {
