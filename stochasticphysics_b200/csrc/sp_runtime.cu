@@ -221,16 +221,25 @@ void* Ensemble::dalloc(size_t bytes) {
 // arithmetic, so the results are bit-identical) into a chunk-sized buffer that the
 // injected step kernel stages like caller-supplied increments.
 //
-// Up to how many particles per SM the separate draw wins (measured, us per step drawn before /
-// in the step): Brown+Neel Euler/spherical to the two warps per scheduler its unbound kernel
-// can have (37888 particles, Heun 3.27 / 3.77), the implicit steps alike; Neel Heun 20001
-// particles 0.77 / 0.82, 30011 0.91 / 0.83; Neel spherical Euler-Maruyama 20001 1.05 / 1.13, 30011
-// 1.24 / 1.17; Brown+Neel Cartesian Heun, whose six draws hide behind its own step, 4096
-// particles 0.78 / 0.87, 9000 0.90 / 0.87.
+// Up to how many particles per SM the separate draw wins (148 SMs; us per step drawn before the
+// chunk / in the step kernel, on both sides of the line):
+//   Neel              Heun 22000 particles 0.69 / 0.76, 30011 0.82 / 0.76
+//   Neel spherical    Euler-Maruyama 30011 1.13 / 1.19, 34000 1.20 / 1.19 (Heun wins to 37888)
+//   Brown+Neel Euler  Heun 37888 3.29 / 3.35; Millstein 30011 2.16 / 2.19, 34000 2.29 / 2.18
+//   Brown+Neel Cart.  Heun 7500 0.774 / 0.791, 10000 0.83 / 0.79 (its draws hide behind the
+//                     step); Millstein 14000 0.83 / 0.87, 18900 0.93 / 0.87
+//   implicit          cubic, 37888: 13.3 / 13.6, exact matrix 4.7 / 5.1
+// Never above two warps per scheduler, 256 per SM, all that the unbound kernels can have.
 constexpr unsigned long long kPregenBytes = 256ull << 20;  // cap on the chunk's increments buffer
 static unsigned long long pregen_particles_per_sm(const sp_ensemble_desc& d) {
-    if (d.solver == SP_SOLVER_IMPLICIT_MIDPOINT || d.problem == SP_PROBLEM_BROWN_AND_NEEL_EULER_SPHERICAL) return 8 * 32;
-    return d.problem == SP_PROBLEM_BROWN_AND_NEEL ? 3 * 16 : 5 * 32;
+    if (d.solver == SP_SOLVER_IMPLICIT_MIDPOINT) return 256;
+    const bool heun = d.solver == SP_SOLVER_HEUN_STRONG;
+    switch (d.problem) {
+        case SP_PROBLEM_NEEL: return 176;
+        case SP_PROBLEM_NEEL_SPHERICAL: return 224;
+        case SP_PROBLEM_BROWN_AND_NEEL_EULER_SPHERICAL: return heun ? 256 : 208;
+        default: return d.solver == SP_SOLVER_MILLSTEIN ? 100 : 56;
+    }
 }
 
 static bool pregen_wanted(const sp_context* ctx, const sp_ensemble_desc& d) {
