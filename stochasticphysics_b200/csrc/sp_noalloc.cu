@@ -102,7 +102,7 @@ extern "C" SP_API sp_status sp_simulate_noalloc(const sp_ensemble_desc* desc, co
         sp_context c;
         c.device = device;
         check_cuda(cudaDeviceGetAttribute(&c.sms, cudaDevAttrMultiProcessorCount, device), "cudaDeviceGetAttribute");
-        const LaunchConfig lc = default_launch(&c, *desc);
+        LaunchConfig lc = default_launch(&c, *desc);
         const EnsembleLayout L = layout_of(*desc, lc);
         const KernelSet& ks = kernel_set(desc->problem, desc->anisotropy, solver_slot(desc->solver, desc->jacobian),
                                          desc->precision, 0);
@@ -110,14 +110,18 @@ extern "C" SP_API sp_status sp_simulate_noalloc(const sp_ensemble_desc* desc, co
 
         // carve the scratch
         const size_t R = L.real;
-        const int ntiles = static_cast<int>((L.n + lc.block - 1) / lc.block);
         size_t off = 0;
         auto take = [&](size_t bytes) { const size_t at = off; off += align256(bytes); return at; };
-        const size_t o_ens = take(sizeof(EnsDev)), o_ctl = take(sizeof(EnsCtl)), o_tiles = take(ntiles * sizeof(TileDesc));
+        const size_t o_ens = take(sizeof(EnsDev)), o_ctl = take(sizeof(EnsCtl));
         const size_t o_state = take(L.Np * L.D * R), o_ksum = take(L.Np * L.OUT * R), o_kcomp = take(L.Np * L.OUT * R);
         const size_t o_slo = R == 4 ? take(L.Np * L.D * R) : 0;
         const size_t o_params = take(L.Np * L.P * R), o_moment = take(L.Np * 8), o_status = take(L.Np);
         const size_t o_partial = take((L.Np / 32) * L.slots * L.OUT * 8), o_ftab = take(L.chunk * 3 * R);
+        // the tile list last, with larger tiles where it would not fit
+        auto tiles_of = [&](int block) { return static_cast<int>((L.n + block - 1) / block); };
+        while (lc.block < kMaxBlock && off + align256(tiles_of(lc.block) * sizeof(TileDesc)) > kNoAllocScratchBytes) lc.block *= 2;
+        const int ntiles = tiles_of(lc.block);
+        const size_t o_tiles = take(ntiles * sizeof(TileDesc));
         if (off > kNoAllocScratchBytes)
             return fail(SP_ERR_INVALID_ARG, "ensemble needs " + std::to_string(off) + " bytes of scratch; the static scratch of "
                                                 "sp_simulate_noalloc holds " + std::to_string(kNoAllocScratchBytes) + " bytes");
