@@ -3,6 +3,8 @@
 
 #include <cuda_runtime.h>
 
+#include <mutex>
+
 #include "sp_types.h"
 
 namespace sp {
@@ -19,7 +21,8 @@ struct KernelSet {
     const void* step_fn[2] = {nullptr, nullptr};  // for cudaFuncGetAttributes / occupancy queries
     // dynamic shared memory of a step launch of `threads` threads (injected increments'
     // staging; 0 for in-kernel noise), and the once-per-device opt-in it needs above the
-    // default limit: call prepare() with the device current before the first launch
+    // default limit: call prepare() with the device current before the first launch (throws
+    // where the device refuses it: the launches would be refused one by one)
     size_t (*dyn_smem)(int threads) = nullptr;
     void (*prepare)() = nullptr;
     // injected-noise sets of solvers with one draw per step: the pregenerated-noise kernel
@@ -42,6 +45,14 @@ inline int solver_slot(int solver, int jacobian) {
     if (solver == kImplicitMidpoint && jacobian == 1) return kImplicitMidpointExact;
     return solver >= 5 ? solver + 1 : solver;
 }
+
+// devices a once-per-device setting has been made on
+struct DeviceOnce {
+    std::mutex mu;
+    bool done[64] = {};
+};
+// opts `kernel` in to launches of `bytes` of dynamic shared memory on the current device
+void allow_dynamic_smem(const void* kernel, size_t bytes, DeviceOnce& once);
 
 void fill_neel(KernelSet* tab);
 void fill_neel_spherical(KernelSet* tab);

@@ -1,8 +1,6 @@
 // sp_instantiate.cuh — builds the KernelSet entries of one problem.
 #pragma once
 
-#include <mutex>
-
 #include "sp_dispatch.h"
 #include "sp_kernels.cuh"
 
@@ -26,20 +24,13 @@ void launch_step_t(const EnsDev* e, const TileDesc* t, int ntiles, int grid, int
     const size_t dyn = F == kCopied ? inj_smem_t<PROB, R, A>(block / PPT) : (F == kDrawn ? drawn_smem_t<PROB, R, A, SOLVER>(block / PPT) : 0);
     step_kernel<PROB, R, A, SOLVER, F, PPT><<<grid, block / PPT, dyn, s>>>(e, t, ntiles);
 }
-// the injected kernels' staging exceeds the default dynamic shared memory limit: raise it
-// once per device for the largest CTA
+// the ring kernels' shared memory exceeds the default dynamic limit: raise it once per device
+// for the largest CTA
 template <int PROB, class R, int A, int SOLVER, int F>
 void prepare_ring_t() {
-    static std::mutex mu;
-    static bool done[64] = {};
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return;
-    std::lock_guard<std::mutex> lk(mu);
-    if (done[dev]) return;
-    if (cudaFuncSetAttribute(reinterpret_cast<const void*>(&step_kernel<PROB, R, A, SOLVER, F, 1>),
-                             cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(F == kCopied ? inj_smem_t<PROB, R, A>(kMaxBlock) : drawn_smem_t<PROB, R, A, SOLVER>(kMaxBlock))) == cudaSuccess)
-        done[dev] = true;
+    static DeviceOnce once;
+    allow_dynamic_smem(reinterpret_cast<const void*>(&step_kernel<PROB, R, A, SOLVER, F, 1>),
+                       F == kCopied ? inj_smem_t<PROB, R, A>(kMaxBlock) : drawn_smem_t<PROB, R, A, SOLVER>(kMaxBlock), once);
 }
 template <int PROB, class R, int A, int SOLVER>
 void launch_noise_t(const EnsDev* e, int n_ens, int grid, cudaStream_t s) {

@@ -161,6 +161,7 @@ extern "C" SP_API sp_status sp_simulate_noalloc(const sp_ensemble_desc* desc, co
         EnsDev* d_ens = reinterpret_cast<EnsDev*>(base + o_ens);
         TileDesc* d_tiles = reinterpret_cast<TileDesc*>(base + o_tiles);
 
+        if (ks.prepare) ks.prepare();
         // the array keeps the previous call's contents: clear the control block and the outputs
         check_cuda(cudaMemsetAsync(e.ctl, 0, sizeof(EnsCtl), s), "clear control block");
         check_cuda(cudaMemsetAsync(device_mean, 0, L.K * L.OUT * 8, s), "clear mean");
@@ -175,7 +176,6 @@ extern "C" SP_API sp_status sp_simulate_noalloc(const sp_ensemble_desc* desc, co
         rp.K2 = dp.cubic_constant; rp.urot = dp.uniaxial_rotation;
         rp.temperature = desc->temperature;
         rp.simple_model = desc->problem_settings.use_simple_model;
-        if (ks.prepare) ks.prepare();
         ks.init(d_ens, rp, L.Np, s);
         ks.reduce(d_ens, 1, 2, 1, s);
         launches_add(3);  // descriptor and tiles, init, reduce

@@ -29,6 +29,7 @@ Error::Error(sp_status s, const std::string& m) : std::runtime_error(m), status(
 
 void check_cuda(cudaError_t e, const char* what) {
     if (e == cudaSuccess) return;
+    cudaGetLastError();  // reported here, not found again by the next check
     const sp_status s = (e == cudaErrorMemoryAllocation) ? SP_ERR_OUT_OF_MEMORY : SP_ERR_CUDA;
     throw Error(s, std::string(what) + ": " + cudaGetErrorString(e));
 }
@@ -51,6 +52,17 @@ double double_noise_rho(int p) {
     double s = 0.0;
     for (int r = 1; r <= p; ++r) s += 1.0 / (static_cast<double>(r) * r);
     return std::sqrt(1.0 / 12.0 - s / (2.0 * kPi * kPi));
+}
+
+void allow_dynamic_smem(const void* kernel, size_t bytes, DeviceOnce& once) {
+    int dev = 0;
+    check_cuda(cudaGetDevice(&dev), "cudaGetDevice");
+    const bool kept = dev >= 0 && dev < static_cast<int>(sizeof(once.done));
+    std::lock_guard<std::mutex> lk(once.mu);
+    if (kept && once.done[dev]) return;
+    check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)),
+               "dynamic shared memory of the step kernel");
+    if (kept) once.done[dev] = true;
 }
 
 // the largest x with sqrt(x) <= tol: comparing x itself gives the same answer without the root
@@ -250,7 +262,7 @@ static bool pregen_wanted(const sp_context* ctx, const sp_ensemble_desc& d) {
 }
 
 Ensemble::Ensemble(sp_context* c, const sp_ensemble_desc& d, const LaunchConfig& lc, bool chunk_graph, bool pregen_ok)
-    : ctx(c), desc(d), launch(lc) {
+    : Ensemble(c, d, lc, Members{}) {  // from here on an exception runs the destructor
     pregen = pregen_ok && pregen_wanted(c, d);
     ks = &kernel_set(d.problem, d.anisotropy, solver_slot(d.solver, d.jacobian), d.precision,
                      (d.noise == SP_NOISE_INJECTED || pregen) ? 1 : 0);
@@ -263,6 +275,7 @@ Ensemble::Ensemble(sp_context* c, const sp_ensemble_desc& d, const LaunchConfig&
     L = layout_of(d, launch);
     if (pregen) L.bytes += L.chunk * L.Mn * L.Np * L.real;
     check_cuda(cudaSetDevice(ctx->device), "cudaSetDevice");
+    if (ks->prepare) ks->prepare();
     check_cuda(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking), "cudaStreamCreate");
     check_cuda(cudaEventCreate(&ev0), "cudaEventCreate");
     check_cuda(cudaEventCreate(&ev1), "cudaEventCreate");
@@ -337,7 +350,6 @@ Ensemble::Ensemble(sp_context* c, const sp_ensemble_desc& d, const LaunchConfig&
     if (pregen)
         noise_grid = static_cast<int>(std::min<unsigned long long>((L.chunk * L.n + 255) / 256,
                                                                    8ull * static_cast<unsigned long long>(ctx->sms)));
-    if (ks->prepare) ks->prepare();
     if (launch.persistent) {
         int per_sm = 0;
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ks->step_fn[ppt - 1], block / ppt,
@@ -472,14 +484,23 @@ void Ensemble::enqueue_chunk(cudaStream_t s) {
     ks->step[ppt - 1](d_ens, d_tiles, ntiles, grid, block, s);
     ks->reduce(d_ens, 1, L.slots, 0, s);
     launch_commit(d_ens, 1, s);
+    // a refused launch shows here and nowhere later: the commit would count its steps as done
+    check_cuda(cudaGetLastError(), "chunk launches");
 }
 
 void Ensemble::build_graph() {
     cudaStream_t cs;
     check_cuda(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking), "capture stream");
     check_cuda(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal), "begin capture");
-    enqueue_chunk(cs);
     cudaGraph_t g = nullptr;
+    try {
+        enqueue_chunk(cs);
+    } catch (...) {
+        cudaStreamEndCapture(cs, &g);
+        if (g) cudaGraphDestroy(g);
+        cudaStreamDestroy(cs);
+        throw;
+    }
     const cudaError_t ce = cudaStreamEndCapture(cs, &g);
     cudaStreamDestroy(cs);
     check_cuda(ce, "end capture");

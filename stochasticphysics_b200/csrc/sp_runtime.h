@@ -128,6 +128,8 @@ struct Ensemble {
     Ensemble(sp_context* c, const sp_ensemble_desc& d, const LaunchConfig& lc, bool chunk_graph = true,
              bool pregen_ok = true);
     ~Ensemble();
+    struct Members {};
+    Ensemble(sp_context* c, const sp_ensemble_desc& d, const LaunchConfig& lc, Members) : ctx(c), desc(d), launch(lc) {}
     Ensemble(const Ensemble&) = delete;
     Ensemble& operator=(const Ensemble&) = delete;
 

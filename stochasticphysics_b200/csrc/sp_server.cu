@@ -275,8 +275,10 @@ struct sp_server {
         g.ks->step[ppt - 1](g.d_ens, g.d_tiles, g.ntiles, g.ntiles, g.block, cs);
         g.ks->reduce(g.d_ens, n, g.max_slots, 0, cs);
         launch_commit(g.d_ens, n, cs);
+        const cudaError_t le = cudaGetLastError();  // a refused launch leaves its node out
         const cudaError_t ce = cudaStreamEndCapture(cs, &g.graph);
         cudaStreamDestroy(cs);
+        check_cuda(le, "chunk launches");
         check_cuda(ce, "end capture");
         check_cuda(cudaGraphInstantiate(&g.gexec, g.graph, 0), "instantiate");
         g.dirty = false;
