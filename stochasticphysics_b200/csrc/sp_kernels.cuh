@@ -436,7 +436,8 @@ __global__ void __launch_bounds__(kMaxBlock / PPT, (step_min_blocks<PROB, R, SOL
         const unsigned long long Np = e.Np, W = e.W;
         // Lanes past the ensemble's end run the last particle's steps and store nothing, which
         // saves a branch around each step (kSkipIdle: kept where it costs registers instead, and
-        // where idle lanes would count Newton iterations).
+        // where idle lanes would count Newton iterations).  A second particle past the end is
+        // skipped: often the whole warp has none.
         if (td.first + (threadIdx.x & ~31u) >= e.n) continue;  // a warp with none; no CTA barrier in this loop
         constexpr bool kImplicit = SOLVER == kImplicitMidpoint || SOLVER == kImplicitMidpointExact;
         constexpr bool kSkipIdle = NOISE == kDrawn || kImplicit;
@@ -452,7 +453,7 @@ __global__ void __launch_bounds__(kMaxBlock / PPT, (step_min_blocks<PROB, R, SOL
         for (int k = 0; k < PPT; ++k) {
             p[k] = td.first + static_cast<unsigned long long>(k) * blockDim.x + threadIdx.x;
             active[k] = p[k] < e.n;
-            pe[k] = active[k] ? p[k] : e.n - 1;
+            pe[k] = source_particle(td.first, blockDim.x, threadIdx.x, k, e.n);
         }
         const double dt_d = e.dt;
         const R dt = static_cast<R>(dt_d);
@@ -531,7 +532,7 @@ __global__ void __launch_bounds__(kMaxBlock / PPT, (step_min_blocks<PROB, R, SOL
                 const unsigned long long g = s0 + t0 + i;
 #pragma unroll
                 for (int k = 0; k < PPT; ++k) {
-                    if (kSkipIdle && !active[k]) continue;
+                    if ((kSkipIdle || k > 0) && !active[k]) continue;
                     [[maybe_unused]] const unsigned long long pid = (kKeepOffset ? kept_offset : e.pid_offset) + p[k];
                     R w[Mn];
                     if constexpr (kRing) {

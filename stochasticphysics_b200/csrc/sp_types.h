@@ -60,6 +60,18 @@ constexpr unsigned char kNonFinite = 1, kChartBrown = 2, kChartNeel = 4;
 // ensemble's dw into a shared-memory ring; drawn into that ring a few steps at a time
 enum NoiseForm : int { kInline = 0, kCopied = 1, kDrawn = 2 };
 
+// The particle that the k-th chain of a thread loads, in a tile that starts at `first` and puts
+// `threads` particles side by side: its own, or, past the ensemble's end, the last one that its
+// warp's first chains hold (the warp's own, so that no other warp can be storing it).  Only for
+// warps whose first chains hold a particle.
+__host__ __device__ inline unsigned long long source_particle(unsigned long long first, unsigned int threads,
+                                                              unsigned int thread, int k, unsigned long long n) {
+    const unsigned long long own = first + static_cast<unsigned long long>(k) * threads + thread;
+    if (own < n) return own;
+    const unsigned long long front = first + thread;
+    return front < n ? front : n - 1;
+}
+
 struct FieldParams {
     int type;  // sp_field_type
     int pad;
