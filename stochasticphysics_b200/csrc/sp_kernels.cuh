@@ -441,8 +441,19 @@ __global__ void __launch_bounds__(kMaxBlock / PPT, (step_min_blocks<PROB, R, SOL
         if (td.first + (threadIdx.x & ~31u) >= e.n) continue;  // a warp with none; no CTA barrier in this loop
         constexpr bool kImplicit = SOLVER == kImplicitMidpoint || SOLVER == kImplicitMidpointExact;
         constexpr bool kSkipIdle = NOISE == kDrawn || kImplicit;
-        unsigned long long p[PPT], pe[PPT];
-        bool active[PPT];
+        // Where chart rotations diverge, an idle lane must not wander to a pole by itself: its warp
+        // would wait for it (Euler-Maruyama, idle lanes on noise of their own: Neel spherical, 1000
+        // particles, 0.68 us per step, now 0.44; Brown+Neel, 3 particles, 0.90, now 0.70).  Neel
+        // spherical: it starts from NaN, for which no threshold holds.  Brown+Neel and the
+        // double-noise solvers, whose divisions and roots take a slow path for NaN (spherical
+        // WeakTest, 37 particles: 1.28, followed 0.98): it follows the last particle's noise, for a
+        // few registers (spherical Heun, 30011: 0.67, from NaN 0.61).
+        constexpr bool kRotating = NOISE == kInline && !kSkipIdle && (PROB == kNeelSpherical || PROB == kBrownNeelEuler);
+        constexpr bool kStartNaN = kRotating && PROB == kNeelSpherical && !uses_double_noise(SOLVER);
+        constexpr bool kFollow = kRotating && !kStartNaN;
+        unsigned long long own[PPT], pe[PPT];
+        bool own_active[PPT];
+        [[maybe_unused]] unsigned int followed[PPT];  // whose noise (kFollow)
         // A load through e inside the step loop is repeated every step (the window stores might
         // alias it).  The Cartesian problems keep the offset (FP32 Neel Heun, 65536 particles:
         // 0.734 -> 0.711 us per step); the angle problems lack the two registers (FP32 Neel
@@ -451,10 +462,21 @@ __global__ void __launch_bounds__(kMaxBlock / PPT, (step_min_blocks<PROB, R, SOL
         const unsigned long long kept_offset = kKeepOffset ? e.pid_offset : 0ull;
 #pragma unroll
         for (int k = 0; k < PPT; ++k) {
-            p[k] = td.first + static_cast<unsigned long long>(k) * blockDim.x + threadIdx.x;
-            active[k] = p[k] < e.n;
+            own[k] = td.first + static_cast<unsigned long long>(k) * blockDim.x + threadIdx.x;
+            own_active[k] = own[k] < e.n;
             pe[k] = source_particle(td.first, blockDim.x, threadIdx.x, k, e.n);
+            followed[k] = static_cast<unsigned int>(pe[k]);  // n <= 2^31
         }
+        // The thread's k-th place in the ensemble, and whether there is such a particle.  Followers
+        // ask the tile list again: kept across the steps these cost registers they do not have.
+        const auto p = [&](int k) {
+            if constexpr (kFollow) return tiles[t].first + static_cast<unsigned long long>(k) * blockDim.x + threadIdx.x;
+            else return own[k];
+        };
+        const auto active = [&](int k) {
+            if constexpr (kFollow) return p(k) < e.n;
+            else return own_active[k];
+        };
         const double dt_d = e.dt;
         const R dt = static_cast<R>(dt_d);
         const R sqdt = static_cast<R>(e.sqrt_dt);
@@ -493,7 +515,10 @@ __global__ void __launch_bounds__(kMaxBlock / PPT, (step_min_blocks<PROB, R, SOL
                 const R* ks = static_cast<const R*>(e.ksum);
                 const R* kc = static_cast<const R*>(e.kcomp);
 #pragma unroll
-                for (int i = 0; i < D; ++i) y[k][i] = state[i * Np + pe[k]];
+                for (int i = 0; i < D; ++i) {
+                    y[k][i] = state[i * Np + pe[k]];
+                    if (kStartNaN && !own_active[k]) y[k][i] = __int_as_float(0x7fffffff);
+                }
 #pragma unroll
                 for (int c = 0; c < OUT; ++c) acc[k].set(c, ks[c * Np + pe[k]], kc[c * Np + pe[k]]);
                 if constexpr (kSharedPar == 0) q[k] = Prob::load(static_cast<const R*>(e.params), Np, pe[k]);
@@ -532,8 +557,8 @@ __global__ void __launch_bounds__(kMaxBlock / PPT, (step_min_blocks<PROB, R, SOL
                 const unsigned long long g = s0 + t0 + i;
 #pragma unroll
                 for (int k = 0; k < PPT; ++k) {
-                    if ((kSkipIdle || k > 0) && !active[k]) continue;
-                    [[maybe_unused]] const unsigned long long pid = (kKeepOffset ? kept_offset : e.pid_offset) + p[k];
+                    if ((kSkipIdle || k > 0) && !own_active[k]) continue;
+                    [[maybe_unused]] const unsigned long long pid = (kKeepOffset ? kept_offset : e.pid_offset) + (kFollow ? followed[k] : own[k]);
                     R w[Mn];
                     if constexpr (kRing) {
 #pragma unroll
@@ -570,22 +595,22 @@ __global__ void __launch_bounds__(kMaxBlock / PPT, (step_min_blocks<PROB, R, SOL
                     double* const traj = e.traj;
 #pragma unroll
                     for (int k = 0; k < PPT; ++k) {
-                        const double mom = active[k] ? e.moment[p[k]] : 0.0;
-                        double* const partial = e.partial + ((p[k] >> 5) * e.slots + slot) * OUT;
+                        const double mom = active(k) ? e.moment[p(k)] : 0.0;
+                        double* const partial = e.partial + ((p(k) >> 5) * e.slots + slot) * OUT;
                         // recorded particles: every traj_stride-th (the reference's Save_intervall)
-                        const bool rec = traj && active[k] && (p[k] + 1) % e.traj_stride == 0;
-                        const unsigned long long ti = rec ? (p[k] + 1) / e.traj_stride - 1 : 0;
+                        const bool rec = traj && active(k) && (p(k) + 1) % e.traj_stride == 0;
+                        const unsigned long long ti = rec ? (p(k) + 1) / e.traj_stride - 1 : 0;
                         // the butterfly leaves every lane with the same sums; lane c keeps
                         // component c, and the warp writes its OUT sums in one coalesced store
                         const int lane = threadIdx.x & 31;
                         double mine = 0.0;
 #pragma unroll
                         for (int c = 0; c < OUT; ++c) {
-                            const R v = active[k] ? acc[k].get_sum(c) / static_cast<R>(static_cast<double>(W)) : R(0);
+                            const R v = active(k) ? acc[k].get_sum(c) / static_cast<R>(static_cast<double>(W)) : R(0);
                             acc[k].clear_sum(c);
                             const double vd = static_cast<double>(v);
                             if (rec) traj[(kw * OUT + c) * e.traj_n + ti] = vd;
-                            const double ws = warp_sum(active[k] ? weight_of<PROB>(c, mom) * vd : 0.0);
+                            const double ws = warp_sum(active(k) ? weight_of<PROB>(c, mom) * vd : 0.0);
                             if (lane == c) mine = ws;
                         }
                         if (lane < OUT) partial[lane] = mine;
@@ -595,7 +620,7 @@ __global__ void __launch_bounds__(kMaxBlock / PPT, (step_min_blocks<PROB, R, SOL
             // own whose independent pairs interleave, instead of inside the step's chain
             [[maybe_unused]] auto draw = [&](R* first, unsigned long long j, int steps) {
                 if constexpr (NOISE == kDrawn) {
-                    const unsigned long long pid = e.pid_offset + p[0];
+                    const unsigned long long pid = e.pid_offset + own[0];
                     for (int st = 0; st < steps; ++st) {
                         R w[Mn];
                         philox_increments<R, Mn>(seed, pid, s0 + j + st, m2dt, w);
@@ -653,26 +678,26 @@ __global__ void __launch_bounds__(kMaxBlock / PPT, (step_min_blocks<PROB, R, SOL
         }
 #pragma unroll
         for (int k = 0; k < PPT; ++k) {
-            if (active[k]) {
+            if (active(k)) {
                 R* state = static_cast<R*>(e.state);
                 R* ks = static_cast<R*>(e.ksum);
                 R* kc = static_cast<R*>(e.kcomp);
                 bool finite = true;
 #pragma unroll
                 for (int i = 0; i < D; ++i) {
-                    state[i * Np + p[k]] = y[k][i];
+                    state[i * Np + p(k)] = y[k][i];
                     finite = finite && M<R>::finite(y[k][i]);
                 }
                 if (e.slo) {
                     R* slo = static_cast<R*>(e.slo);
 #pragma unroll
-                    for (int i = 0; i < D; ++i) slo[i * Np + p[k]] = lo[k][i];
+                    for (int i = 0; i < D; ++i) slo[i * Np + p(k)] = lo[k][i];
                 }
 #pragma unroll
-                for (int c = 0; c < OUT; ++c) { ks[c * Np + p[k]] = acc[k].get_sum(c); kc[c * Np + p[k]] = acc[k].get_comp(c); }
+                for (int c = 0; c < OUT; ++c) { ks[c * Np + p(k)] = acc[k].get_sum(c); kc[c * Np + p(k)] = acc[k].get_comp(c); }
                 if constexpr (Prob::kCarriedChart)
-                    e.status[p[k]] = static_cast<unsigned char>((e.status[p[k]] & kNonFinite) | (finite ? 0 : kNonFinite) | Prob::chart_bits(tr[k]));
-                else if (!finite) e.status[p[k]] = kNonFinite;
+                    e.status[p(k)] = static_cast<unsigned char>((e.status[p(k)] & kNonFinite) | (finite ? 0 : kNonFinite) | Prob::chart_bits(tr[k]));
+                else if (!finite) e.status[p(k)] = kNonFinite;
             }
         }
         if constexpr (SOLVER == kImplicitMidpoint || SOLVER == kImplicitMidpointExact) {
