@@ -440,7 +440,12 @@ __global__ void __launch_bounds__(kMaxBlock / PPT, (step_min_blocks<PROB, R, SOL
         // skipped: often the whole warp has none.
         if (td.first + (threadIdx.x & ~31u) >= e.n) continue;  // a warp with none; no CTA barrier in this loop
         constexpr bool kImplicit = SOLVER == kImplicitMidpoint || SOLVER == kImplicitMidpointExact;
-        constexpr bool kSkipIdle = NOISE == kDrawn || kImplicit;
+        // The longest FP32 Brown+Neel steps are skipped too: one block of code takes
+        // Heun_NotConsistent to 154 registers, 12 warps per SM, with the branch it stays at 128
+        // (70001 particles: 4.83 us per step, skipping 4.11; uniaxial+cubic Heun, 37: 1.44, 1.35).
+        constexpr bool kSkipIdle = NOISE == kDrawn || kImplicit ||
+                                   (PROB == kBrownNeelEuler && NOISE == kInline &&
+                                    (SOLVER == kHeunNotConsistent || (A == kUniaxialCubic && SOLVER == kHeun)));
         // Where chart rotations diverge, an idle lane must not wander to a pole by itself: its warp
         // would wait for it (Euler-Maruyama, idle lanes on noise of their own: Neel spherical, 1000
         // particles, 0.68 us per step, now 0.44; Brown+Neel, 3 particles, 0.90, now 0.70).  Neel
