@@ -650,9 +650,11 @@ __global__ void __launch_bounds__(kMaxBlock / PPT, (step_min_blocks<PROB, R, SOL
                     if constexpr (kRuns) run = min(run, dws.left());
                     rows = dws.rows() + column;
                 }
-                // a Neel step is short enough for four to be scheduled as one (1024 particles,
-                // Heun: 0.353 us per step one at a time, 0.342 by fours; longer steps gain nothing)
-                constexpr int kUnroll = NOISE == kCopied && PROB == kNeel && SOLVER != kImplicitMidpoint && SOLVER != kImplicitMidpointExact ? 4 : 1;
+                // Short steps are scheduled several as one (1024 Neel particles, Heun: 0.353 us per
+                // step one at a time, 0.342 by fours; 32 Brown+Neel Cartesian ones, Euler-Maruyama:
+                // 0.580, a stage of five 0.527).  Longer steps gain nothing.
+                constexpr bool kEuler = SOLVER == kEulerMaruyama || SOLVER == kEulerMaruyamaNormalized;
+                constexpr int kUnroll = NOISE != kCopied || kImplicit ? 1 : PROB == kNeel ? 4 : PROB == kBrownNeel && kEuler ? 5 : 1;
 #pragma unroll kUnroll
                 for (int j = 0; j < run; ++j) {
                     const R B[3] = {sB[i + j][0], sB[i + j][1], sB[i + j][2]};
