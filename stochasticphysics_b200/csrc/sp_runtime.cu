@@ -226,31 +226,44 @@ void* Ensemble::dalloc(size_t bytes) {
 
 // Pregenerated noise.  A small ensemble leaves most SMs idle and each step's time is the
 // latency of one thread's step chain, in which the FP64 Philox draw and Box-Muller pairs
-// lengthen the chain (Neel Heun, 1024 particles: 0.67 us per step with in-kernel noise, 0.43
-// with the increments read from memory; Brown+Neel Heun 3.12 and 1.70).  With at most two
+// lengthen the chain (4000 particles: Neel Heun 0.615 us per step with in-kernel noise, 0.391
+// with the increments read from memory; Brown+Neel Euler Heun 2.66 and 1.66).  With at most two
 // warps per SM scheduler, an FP64 ensemble with in-kernel noise therefore draws each chunk's
 // increments in a separate, fully parallel kernel (the same Philox counters and
 // arithmetic, so the results are bit-identical) into a chunk-sized buffer that the
 // injected step kernel stages like caller-supplied increments.
 //
-// Up to how many particles per SM the separate draw wins (148 SMs; us per step drawn before the
-// chunk / in the step kernel, on both sides of the line):
-//   Neel              Heun 22000 particles 0.69 / 0.76, 30011 0.82 / 0.76
-//   Neel spherical    Euler-Maruyama 30011 1.13 / 1.19, 34000 1.20 / 1.19 (Heun wins to 37888)
-//   Brown+Neel Euler  Heun 37888 3.29 / 3.35; Millstein 30011 2.16 / 2.19, 34000 2.29 / 2.18
-//   Brown+Neel Cart.  Heun 7500 0.774 / 0.791, 10000 0.83 / 0.79 (its draws hide behind the
-//                     step); Millstein 14000 0.83 / 0.87, 18900 0.93 / 0.87
+// Up to how many particles per SM the separate draw wins, by the step's length: the longer the
+// step, the better it hides the draw inside it (148 SMs; us per step drawn before the chunk / in
+// the step kernel, on both sides of the line):
+//   Neel              Heun 22000 particles 0.692 / 0.756, 26500 0.761 / 0.757; Euler-Maruyama 26500
+//                     0.656 / 0.715, 30011 0.727 / 0.721; cubic Heun 22000 0.773 / 0.800, 24500
+//                     0.817 / 0.801 (one warp per scheduler, 16000 to 18944, 0.65 / 0.61)
+//   Neel spherical    Euler-Maruyama 33000 1.159 / 1.221, 37888 1.254 / 1.244; cubic 30011 1.188 /
+//                     1.217, 35000 1.272 / 1.214; uniaxial+cubic 37888 1.324 / 1.334
+//   Brown+Neel Euler  Heun 37888 3.27 / 3.33; Millstein 30011 2.17 / 2.18, 33000 2.24 / 2.19;
+//                     Euler-Maruyama 30011 2.22 / 2.21; uniaxial+cubic, whose drawing kernel has
+//                     no room for its prefactors, Euler-Maruyama 37888 2.77 / 2.98
+//   Brown+Neel Cart.  Heun 7500 0.771 / 0.787, 9000 0.813 / 0.788, cubic 10500 0.740 / 0.755,
+//                     12500 0.791 / 0.757; Euler-Maruyama 10500 0.767 / 0.794, 12500 0.815 /
+//                     0.795, cubic 24500 1.031 / 1.069, 26500 1.076 / 1.069; Millstein 14000
+//                     0.836 / 0.866, 18900 0.943 / 0.870, cubic 24500 1.056 / 1.078, 26500
+//                     1.103 / 1.080
 //   implicit          cubic, 37888: 13.3 / 13.6, exact matrix 4.7 / 5.1
 // Never above two warps per scheduler, 256 per SM, all that the unbound kernels can have.
 constexpr unsigned long long kPregenBytes = 256ull << 20;  // cap on the chunk's increments buffer
 static unsigned long long pregen_particles_per_sm(const sp_ensemble_desc& d) {
     if (d.solver == SP_SOLVER_IMPLICIT_MIDPOINT) return 256;
-    const bool heun = d.solver == SP_SOLVER_HEUN_STRONG;
+    const bool heun = d.solver == SP_SOLVER_HEUN_STRONG, cubic = d.anisotropy != SP_ANISOTROPY_UNIAXIAL,
+               both = d.anisotropy == SP_ANISOTROPY_UNIAXIAL_CUBIC;
     switch (d.problem) {
-        case SP_PROBLEM_NEEL: return 176;
-        case SP_PROBLEM_NEEL_SPHERICAL: return 224;
-        case SP_PROBLEM_BROWN_AND_NEEL_EULER_SPHERICAL: return heun ? 256 : 208;
-        default: return d.solver == SP_SOLVER_MILLSTEIN ? 100 : 56;
+        case SP_PROBLEM_NEEL: return heun && cubic ? 152 : 176;
+        case SP_PROBLEM_NEEL_SPHERICAL: return both ? 256 : 224;
+        case SP_PROBLEM_BROWN_AND_NEEL_EULER_SPHERICAL: return heun || both ? 256 : 208;
+        default:
+            if (heun) return cubic ? 72 : 56;
+            if (cubic) return 168;
+            return d.solver == SP_SOLVER_MILLSTEIN ? 100 : 76;
     }
 }
 
