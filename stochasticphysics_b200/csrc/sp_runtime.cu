@@ -318,7 +318,9 @@ Ensemble::Ensemble(sp_context* c, const sp_ensemble_desc& d, const LaunchConfig&
     // injected increments: [S][M][n] FP64 host -> [S][M][Np] Real device
     if (d.noise == SP_NOISE_INJECTED && L.S > 0) {
         d_dw = dalloc(L.S * L.Mn * L.Np * R);
-        upload_increments(ctx, d.injected_dw, d_dw, L.real, L.S * L.Mn, L.n, L.Np, stream);
+        const unsigned long long spread = upload_increments(ctx, d.injected_dw, d_dw, L.real, L.S * L.Mn, L.n, L.Np, stream);
+        launches += spread;
+        g_launch_count += spread;
     }
 
     // device descriptor

@@ -54,9 +54,10 @@ int noise_dim(int p);
 int out_dim(int p);
 int param_count(int p, int aniso);
 double double_noise_rho(int p);
-// caller-supplied increments [rows][n] (host) -> [rows][Np] of `real` bytes each (sp_upload.cu)
-void upload_increments(sp_context* ctx, const double* src, void* dst, int real, size_t rows, size_t n, size_t Np,
-                       cudaStream_t s);
+// caller-supplied increments [rows][n] (host) -> [rows][Np] of `real` bytes each (sp_upload.cu);
+// returns the kernels it launched
+unsigned long long upload_increments(sp_context* ctx, const double* src, void* dst, int real, size_t rows, size_t n, size_t Np,
+                                     cudaStream_t s);
 double squared_tolerance(double tol);
 FieldParams field_params(const sp_field_desc& f);
 void reference_times(unsigned long long K, unsigned long long W, double dt, double* times);

@@ -88,7 +88,7 @@ const KernelSet& kernel_set(int, int, int, int, int inject) {
 }
 RawParticles provided_raw(const double*, unsigned long long) { return {}; }
 double* provide_particles(sp_context*, const sp_ensemble_desc&, cudaStream_t) { return nullptr; }
-void upload_increments(sp_context*, const double*, void*, int, size_t, size_t, size_t, cudaStream_t) {}
+unsigned long long upload_increments(sp_context*, const double*, void*, int, size_t, size_t, size_t, cudaStream_t) { return 0; }
 void launch_commit(const EnsDev*, int, cudaStream_t) {}
 void launch_bump_targets(const EnsDev*, int, cudaStream_t) {}
 void launch_set_target(EnsCtl*, unsigned long long, cudaStream_t) {}
