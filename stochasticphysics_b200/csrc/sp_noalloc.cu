@@ -133,7 +133,7 @@ extern "C" SP_API sp_status sp_simulate_noalloc(const sp_ensemble_desc* desc, co
         std::memset(&e, 0, sizeof(e));
         e.n = L.n; e.Np = L.Np; e.K = L.K; e.W = L.W; e.S = L.S; e.chunk = L.chunk;
         e.seed = desc->seed; e.pid_offset = desc->particle_id_offset;
-        e.dt = desc->timestep; e.sqrt_dt = std::sqrt(desc->timestep);
+        e.dt = device_step(*desc); e.sqrt_dt = std::sqrt(e.dt);
         e.field = field_params(desc->field);
         e.max_iter = desc->max_iteration; e.tol = R == 8 ? squared_tolerance(desc->accuracy_goal) : desc->accuracy_goal;
         e.dna = desc->double_noise_approx; e.rho = double_noise_rho(desc->double_noise_approx);

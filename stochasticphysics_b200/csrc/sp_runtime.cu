@@ -65,6 +65,13 @@ void allow_dynamic_smem(const void* kernel, size_t bytes, DeviceOnce& once) {
     if (kept) once.done[dev] = true;
 }
 
+// The step the kernels integrate with.  FP64: no shorter than 2^-960 s, below which -2 dt ln u
+// leaves the normal numbers that their square root takes.  Increments of that size (2^-480, and
+// 2^-960 times a rate) are lost in a state of order one either way.
+double device_step(const sp_ensemble_desc& d) {
+    return d.precision == SP_PRECISION_FP64 ? std::max(d.timestep, 0x1p-960) : d.timestep;
+}
+
 // the largest x with sqrt(x) <= tol: comparing x itself gives the same answer without the root
 double squared_tolerance(double tol) {
     const double inf = std::numeric_limits<double>::infinity(), most = std::numeric_limits<double>::max();
@@ -328,7 +335,7 @@ Ensemble::Ensemble(sp_context* c, const sp_ensemble_desc& d, const LaunchConfig&
     std::memset(&e, 0, sizeof(e));
     e.n = L.n; e.Np = L.Np; e.K = L.K; e.W = L.W; e.S = L.S; e.chunk = L.chunk;
     e.seed = d.seed; e.pid_offset = d.particle_id_offset;
-    e.dt = d.timestep; e.sqrt_dt = std::sqrt(d.timestep);
+    e.dt = device_step(d); e.sqrt_dt = std::sqrt(e.dt);
     e.field = field_params(d.field);
     e.max_iter = d.max_iteration; e.tol = R == 8 ? squared_tolerance(d.accuracy_goal) : d.accuracy_goal;
     e.dna = d.double_noise_approx; e.rho = double_noise_rho(d.double_noise_approx);

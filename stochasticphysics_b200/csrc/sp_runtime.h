@@ -59,6 +59,7 @@ double double_noise_rho(int p);
 unsigned long long upload_increments(sp_context* ctx, const double* src, void* dst, int real, size_t rows, size_t n, size_t Np,
                                      cudaStream_t s);
 double squared_tolerance(double tol);
+double device_step(const sp_ensemble_desc& d);
 FieldParams field_params(const sp_field_desc& f);
 void reference_times(unsigned long long K, unsigned long long W, double dt, double* times);
 
