@@ -638,10 +638,11 @@ __global__ void __launch_bounds__(kMaxBlock / PPT, (step_min_blocks<PROB, R, SOL
             // basic block (a branch stops the scheduler from filling the FP64 chains' gaps with the
             // next step's work): Neel Heun, 1024 particles, 0.428 us per step with the checks and an
             // idle-lane branch inside, 0.391 in runs of at most four steps, 0.353 of eight; Neel
-            // spherical Euler-Maruyama 0.737, 0.621, 0.579.  Not where a step is long and the
-            // registers are all taken (Brown+Neel Euler drawing its noise: 3.68 us checked, 3.77
-            // in runs; cubic implicit, 4000 particles: 9.6 and 10.2).
-            constexpr bool kRuns = !kImplicit && (NOISE == kCopied || (NOISE == kInline && PROB != kBrownNeelEuler));
+            // spherical Euler-Maruyama 0.737, 0.621, 0.579.  Neel spherical drawing
+            // its noise, Euler-Maruyama, 65536: 1.84 checked, 1.78 in runs.  Not where a step is
+            // long and the registers are all taken (Brown+Neel Euler drawing its noise, Millstein,
+            // 65536: 3.64 checked, 3.69 in runs; cubic implicit, 4000 particles: 9.6 and 10.2).
+            constexpr bool kRuns = !kImplicit && (NOISE == kCopied || PROB != kBrownNeelEuler);
             for (int i = 0; i < len;) {
                 int run = kRuns ? static_cast<int>(min(static_cast<unsigned int>(len - i), W32 - wpos)) : 1;
                 [[maybe_unused]] const R* rows = nullptr;
