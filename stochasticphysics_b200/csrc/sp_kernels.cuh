@@ -360,18 +360,18 @@ struct WindowSum<float, OUT> {
 // small ensembles, one or two warps per scheduler, where a spill only lengthens the chain:
 // unbound (Brown+Neel Heun, 1024 particles: 1.70 us per step, 2.79 bound).  The
 // implicit-midpoint kernels are bound too (cubic Neel, 262144 particles, reference matrix:
-// 77 us per step, 89 with the 160 registers left alone; exact matrix: 28.5, 16 % faster than
+// 76 us per step, 89 with the 160 registers left alone; exact matrix: 28.2, 16 % faster than
 // unbound).  Register allocation does not change the arithmetic.
 //
 // Where the increments of a kernel with in-kernel noise are drawn (NOISE): inside the step,
 // where the pairs' chains interleave with the step's own (Cartesian problems, FP32 and the
 // implicit steps), or a stage of steps ahead in a loop of its own (kDrawn, the FP64 angle
 // problems), whose steps fill the registers and the instruction cache by themselves
-// (Neel spherical Euler-Maruyama, 65536 particles: 1.85 us per step staged; Brown+Neel
+// (Neel spherical Euler-Maruyama, 65536 particles: 1.78 us per step staged; Brown+Neel
 // Cartesian Heun, whose step is a third of that: 2.51 inside, 2.85 staged).
 // The angle problems' FP64 steps with the library's sines and pairs called one after another
 // and the chart rotated and turned back on every step: Brown+Neel Millstein, 65536 particles,
-// 9.17 us per step, now 3.76; Heun 12.4, now 5.49.
+// 9.17 us per step, now 3.64; Heun 12.4, now 5.40.
 template <int PROB, class R, int SOLVER, int NOISE, int PPT>
 constexpr int step_min_blocks() {
     return (sizeof(R) == 8 && NOISE != kCopied &&

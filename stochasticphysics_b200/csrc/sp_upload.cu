@@ -6,7 +6,8 @@
 // pitch and converts them where the layouts differ (FP32, or n not a multiple of kPad).  The
 // host therefore touches every increment once.  16384 particles, 250 steps (98 MB) on
 // a B200 host: 3.6-4.8 ms; building the padded array on the host first and handing the driver
-// a pageable copy of it took 53-55 ms.  865 MB: 23 ms.  Below 4 MB one thread is as fast.
+// a pageable copy of it took 53-55 ms.  The first upload of a context also allocates the pieces and
+// grows the pool: whole call 22-37 ms there, 4 ms after, 59 and 55 the old way.  865 MB: 23 ms.  Below 4 MB one thread is as fast.
 #include <algorithm>
 #include <cstring>
 #include <numeric>
